@@ -70,8 +70,8 @@ struct DevSide {
     int32_t *val_row = nullptr, *val_col = nullptr;
     int32_t *pat[4] = {};  // pattern row_ptr, col_idx, output_ptr, output_rows
     // row-segment stream (kernel 5): chunks, segment meta, spans, counters,
-    // partial slots, rowmap, empty rows, value positions, window bases
-    void *rs[9] = {};
+    // partial slots, rowmap, empty rows, value positions, window bases, window lengths
+    void *rs[10] = {};
     int64_t rs_bytes = 0;
     std::vector<int32_t> rs_cinfo;  // per chunk summaries (batches cut their own segments)
     std::vector<int32_t> rs_empty;  // rows without entries
@@ -322,6 +322,7 @@ cbspmv_status upload_rowseg(DevSide &s, int kernel, cudaStream_t st) {
     CB_CUDA(upload_vec(R.empty, (int32_t **)&s.rs[6], st), "upload row segments");
     CB_CUDA(upload_vec(R.vpos, (int32_t **)&s.rs[7], st), "upload row segments");
     CB_CUDA(upload_vec(R.wbase, (int32_t **)&s.rs[8], st), "upload row segments");
+    CB_CUDA(upload_vec(R.wlen, (int32_t **)&s.rs[9], st), "upload row segments");
     cb::RowSegDev &d = s.d.rs;
     d.chunks = static_cast<const uint8_t *>(s.rs[0]);
     d.nch = R.nch;
@@ -337,8 +338,10 @@ cbspmv_status upload_rowseg(DevSide &s, int kernel, cudaStream_t st) {
     d.nempty = (int32_t)R.empty.size();
     d.vpos = static_cast<const int32_t *>(s.rs[7]);
     d.G = R.G;
-    d.W = R.W;
+    // (at least one value: the launch asks for the longest window in use)
+    d.W = std::max<int32_t>(1, *std::max_element(R.wlen.begin(), R.wlen.end()));
     d.wbase = static_cast<const int32_t *>(s.rs[8]);
+    d.wlen = static_cast<const int32_t *>(s.rs[9]);
     d.n = R.n;
     d.unit = R.unit;
     d.auto1 = cb::rowseg_all_coo(s.lay) ? 1 : 0;
@@ -1272,6 +1275,7 @@ int64_t export_device(const cb::DeviceLayout &L, const std::string &k, void *out
         if (f == "empty") return raw(R.empty.data(), R.empty.size() * 4, 4);
         if (f == "vpos") return raw(R.vpos.data(), R.vpos.size() * 4, 4);
         if (f == "wbase") return raw(R.wbase.data(), R.wbase.size() * 4, 4);
+        if (f == "wlen") return raw(R.wlen.data(), R.wlen.size() * 4, 4);
     }
     return -1;
 }

@@ -21,8 +21,9 @@ struct RowSegDev {
     const int32_t *empty = nullptr;   // rows without stored entries
     int32_t nempty = 0;
     const int32_t *vpos = nullptr;    // per stored value: its stream entry
-    int32_t G = 0, W = 0;             // CTAs of every launch; window length (values)
+    int32_t G = 0, W = 0;             // CTAs of every launch; longest window (values)
     const int32_t *wbase = nullptr;   // per CTA: first column of its x window
+    const int32_t *wlen = nullptr;    // per CTA: columns of its x window
     int64_t n = 0;                    // columns (length of x)
     int unit = 0;                     // words only: every stored value is 1
     int auto1 = 0;                    // the automatic choice for one right-hand side

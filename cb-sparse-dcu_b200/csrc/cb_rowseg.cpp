@@ -216,39 +216,57 @@ std::string build_rowseg(const DeviceLayout &L, int64_t warps, RowSegHost &R) {
         cuts.push_back(nch);
         rowseg_cut(R.cinfo, cuts, 0, 0, R.meta, R.spans);
     }
-    // the CTAs' windows of x: per CTA, the W consecutive columns holding the
-    // most of its entries (a sliding window over its sorted columns)
+    // the CTAs' windows of x.  A window costs its length in bytes to stage and
+    // saves its entries a 32-byte sector of L2 traffic each, so per CTA the
+    // window of at most W columns with the largest saving minus cost (a
+    // sliding minimum over its sorted columns), aligned down to kRsWinAlign
+    // columns; no window where every one costs more than it saves
     const int64_t G = std::max<int64_t>(1, std::max<int64_t>(warps, 1) / kRsWarps);
     const int64_t W = kRsWindowBytes / vsz;
     R.G = (int32_t)G;
     R.W = (int32_t)W;
     R.wbase.assign((size_t)G, 0);
-    std::vector<int32_t> cols;
-    for (int64_t b = 0; b < G; ++b) {
-        const int64_t s0 = b * nseg / G, s1 = (b + 1) * nseg / G;
-        const int64_t e0 = std::min(nv, s0 * M * C), e1 = std::min(nv, s1 * M * C);
-        if (e0 >= e1) continue;
-        cols.clear();
-        for (int64_t e = e0; e < e1; ++e) cols.push_back(ecol[order[(size_t)e]]);
-        std::sort(cols.begin(), cols.end());
-        size_t best = 0, lo = 0;
-        int32_t wb = cols[0];
-        for (size_t hi = 0; hi < cols.size(); ++hi) {
-            while ((int64_t)cols[hi] - cols[lo] >= W) ++lo;
-            if (hi - lo + 1 > best) {
-                best = hi - lo + 1;
-                wb = cols[lo];
+    R.wlen.assign((size_t)G, 0);
+#pragma omp parallel
+    {
+        std::vector<int32_t> cols;
+        std::vector<size_t> q;  // candidate first entries, their scores increasing
+#pragma omp for schedule(dynamic, 1)
+        for (int64_t b = 0; b < G; ++b) {
+            const int64_t s0 = b * nseg / G, s1 = (b + 1) * nseg / G;
+            const int64_t e0 = std::min(nv, s0 * M * C), e1 = std::min(nv, s1 * M * C);
+            if (e0 >= e1) continue;
+            cols.clear();
+            for (int64_t e = e0; e < e1; ++e) cols.push_back(ecol[order[(size_t)e]]);
+            std::sort(cols.begin(), cols.end());
+            auto score = [&](size_t i) { return kRsSector * (int64_t)i - vsz * cols[i]; };
+            q.clear();
+            size_t qh = 0;
+            int64_t best = 0;
+            int32_t wb = 0, we = 0;  // the window's columns [wb, we)
+            for (size_t hi = 0; hi < cols.size(); ++hi) {
+                while (q.size() > qh && score(q.back()) >= score(hi)) q.pop_back();
+                q.push_back(hi);
+                // (the window's first column moves down to a multiple of kRsWinAlign)
+                while (cols[hi] - (cols[q[qh]] & ~(kRsWinAlign - 1)) >= W) ++qh;
+                const int64_t gain = score(hi) - score(q[qh]) + kRsSector - vsz;
+                if (gain > best) {
+                    best = gain;
+                    wb = cols[q[qh]] & ~(kRsWinAlign - 1);
+                    we = cols[hi] + 1;
+                }
             }
-        }
-        R.wbase[(size_t)b] = wb;
-        for (int64_t e = e0; e < e1; ++e) {
-            const int64_t col = ecol[order[(size_t)e]];
-            if (col >= wb && col < wb + W) {
-                const int64_t c = e / C, i = e % C;
-                uint32_t word;
-                std::memcpy(&word, R.chunks.data() + c * CB + 4 * i, 4);
-                word |= kRsWin;
-                std::memcpy(R.chunks.data() + c * CB + 4 * i, &word, 4);
+            R.wbase[(size_t)b] = wb;
+            R.wlen[(size_t)b] = we - wb;
+            for (int64_t e = e0; e < e1; ++e) {
+                const int32_t col = ecol[order[(size_t)e]];
+                if (col >= wb && col < we) {
+                    const int64_t c = e / C, i = e % C;
+                    uint32_t word;
+                    std::memcpy(&word, R.chunks.data() + c * CB + 4 * i, 4);
+                    word |= kRsWin;
+                    std::memcpy(R.chunks.data() + c * CB + 4 * i, &word, 4);
+                }
             }
         }
     }

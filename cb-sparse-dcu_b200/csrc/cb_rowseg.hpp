@@ -23,9 +23,10 @@
 // partial sum in a slot (2 s: the segment's first row, 2 s + 1: its last),
 // and the last segment to arrive on the span's counter adds the slots in
 // segment order and stores y, so results do not depend on timing.
-// Each CTA also holds a WINDOW of x in shared memory: kRsWindowBytes of
-// consecutive columns from wbase[b], chosen on the host to cover the most
-// entries of the CTA's segments; an entry whose column lies in its CTA's
+// Each CTA also holds a WINDOW of x in shared memory: wlen[b] consecutive
+// columns from wbase[b], at most kRsWindowBytes, chosen on the host as the one
+// that saves the most gather traffic over its own staging (none where every
+// window costs more than it saves); an entry whose column lies in its CTA's
 // window carries bit 30 and reads x from there (a shared-memory gather costs
 // a few wavefronts per warp where 32 scattered global loads cost 32 L1 tag
 // lookups).  The segments are assigned to CTAs for a grid of G CTAs fixed at
@@ -52,6 +53,8 @@ constexpr uint32_t kRsStart = 1u << 31;   // word: the entry starts a row
 constexpr uint32_t kRsWin = 1u << 30;    // word: x[column] is in the CTA's window
 constexpr uint32_t kRsColMask = (1u << 30) - 1;
 constexpr int64_t kRsWindowBytes = int64_t(128) << 10;
+constexpr int32_t kRsWinAlign = 4;   // a window's first column is a multiple (16-byte copies)
+constexpr int64_t kRsSector = 32;    // bytes of L2 traffic of a gather outside the window
 constexpr int64_t kRsMaxCols = int64_t(1) << 30;
 
 inline int rs_chunk_entries() { return 32 * kRsK; }
@@ -77,8 +80,9 @@ struct RowSegHost {
     int32_t nseg = 0;
     int32_t nord = 0;       // non-empty rows
     int32_t G = 0;          // CTAs of every launch
-    int32_t W = 0;          // window length in values
+    int32_t W = 0;          // largest window length in values
     std::vector<int32_t> wbase;    // per CTA: first column of its window
+    std::vector<int32_t> wlen;     // per CTA: columns of its window (0: none)
     // per chunk: ordinal running before its first entry, its first entry
     // starts a row, row starts in it, ordinal of its last entry (what any
     // other segmentation needs: a batch cuts its own)

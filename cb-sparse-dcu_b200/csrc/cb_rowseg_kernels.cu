@@ -98,27 +98,47 @@ __device__ __forceinline__ void rs_arrive(const RowSegDev &rs, T *__restrict__ y
     }
 }
 
-template <typename T, bool UNIT>
+// src[0 .. len) into shared memory by asynchronous copies of the whole CTA:
+// all of a thread's copies are in flight at once and take no registers, so
+// the staging costs one memory latency and its bytes (a load-then-store loop
+// waited for memory once per few values).  16-byte copies when src is aligned
+// to them, else value by value.  stage_wait before the CTA's barrier.
+template <typename T>
+__device__ __forceinline__ void stage_window(T *dst, const T *src, int len, int tid) {
+    constexpr int NV = 16 / sizeof(T);
+    int i0 = 0;
+    if (reinterpret_cast<uintptr_t>(src) % 16 == 0) {
+        for (int i = tid; i < len / NV; i += kRsWarps * 32)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                             dev::smem_u32(dst + i * NV)),
+                         "l"(src + i * NV)
+                         : "memory");
+        i0 = len / NV * NV;
+    }
+    for (int i = i0 + tid; i < len; i += kRsWarps * 32)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dev::smem_u32(dst + i)),
+                     "l"(src + i), "n"((int)sizeof(T))
+                     : "memory");
+}
+__device__ __forceinline__ void stage_wait() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+template <typename T, bool UNIT, bool MAP>
 __global__ void __launch_bounds__(kRsWarps * 32, 1)
     cb_rowseg_kernel(const RowSegDev rs, const T *__restrict__ x, T *__restrict__ y) {
     using V = typename RsVec<T>::V;
     constexpr int K = kRsK, NV = RsVec<T>::n;
     constexpr int64_t CB = 32 * K * (4 + (UNIT ? 0 : (int64_t)sizeof(T)));
     extern __shared__ __align__(16) unsigned char rs_smem[];
-    T *xs = reinterpret_cast<T *>(rs_smem);  // x[wb .. wb + W)
+    T *xs = reinterpret_cast<T *>(rs_smem);  // x[wb .. wb + wl)
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    for (int i = (blockIdx.x * kRsWarps + wib) * 32 + lane; i < rs.nempty;
-         i += gridDim.x * kRsWarps * 32)
-        y[__ldg(&rs.empty[i])] = T(0);
     const int G = gridDim.x, b = blockIdx.x;
-    const int64_t wb = __ldg(&rs.wbase[b]);
-    for (int i = threadIdx.x; i < rs.W; i += kRsWarps * 32)
-        xs[i] = wb + i < rs.n ? __ldg(x + wb + i) : T(0);
-    __syncthreads();
+    const int wb = __ldg(&rs.wbase[b]);
+    const int wl = __ldg(&rs.wlen[b]);
     const int sb0 = (int)((int64_t)b * rs.nseg / G);
     const int sb1 = (int)((int64_t)(b + 1) * rs.nseg / G);
     int s = sb0 + wib;
-    if (s >= sb1) return;
     const int M = rs.M, nch = rs.nch, nord = rs.nord;
     const uint64_t pol = dev::policy_evict_first();
     uint4 nw[K / 4];
@@ -133,9 +153,17 @@ __global__ void __launch_bounds__(kRsWarps * 32, 1)
             for (int q = 0; q < K / NV; ++q) nv[q] = ld_stream(gv + q * 32 + lane, pol);
         }
     };
-    auto rid = [&](int32_t o) { return rs.rowmap ? __ldg(&rs.rowmap[o]) : o; };
+    auto rid = [&](int32_t o) { return MAP ? __ldg(&rs.rowmap[o]) : o; };
+    const uint32_t below = (1u << lane) - 1u;
     int c = s * M;
-    load(c);
+    if (s < sb1) load(c);  // in flight while the window is staged
+    stage_window(xs, x + wb, wl, threadIdx.x);
+    for (int i = (blockIdx.x * kRsWarps + wib) * 32 + lane; i < rs.nempty;
+         i += gridDim.x * kRsWarps * 32)
+        y[__ldg(&rs.empty[i])] = T(0);
+    stage_wait();
+    __syncthreads();
+    if (s >= sb1) return;
     while (true) {
         // segment s: meta = {ordinal running before its first entry, its first
         // entry starts a row, head span, tail span}
@@ -172,18 +200,18 @@ __global__ void __launch_bounds__(kRsWarps * 32, 1)
 #pragma unroll
             for (int j = 0; j < K; ++j) {
                 const uint32_t col = w[j] & kRsColMask;
-                xv[j] = (w[j] & kRsWin) ? xs[col - wb] : __ldg(x + col);
+                xv[j] = (w[j] & kRsWin) ? xs[(int)col - wb] : __ldg(x + col);
             }
-            int cnt = 0;
+            // row starts of the lanes before this one, and the lanes that hold
+            // one, from one ballot per entry
+            uint32_t heads = 0;
+            int32_t ordS = ord0;  // the row this lane starts in
 #pragma unroll
-            for (int j = 0; j < K; ++j) cnt += (int)(w[j] >> 31);
-            int inc = cnt;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int t = __shfl_up_sync(kFull, inc, d);
-                if (lane >= d) inc += t;
+            for (int j = 0; j < K; ++j) {
+                const uint32_t bal = __ballot_sync(kFull, (w[j] >> 31) != 0);
+                heads |= bal;
+                ordS += __popc(bal & below);
             }
-            const int32_t ordS = ord0 + inc - cnt;  // the row this lane starts in
             int32_t ord = ordS;
             T run = T(0), head = T(0);
             bool seen = false;  // a row starts in this lane
@@ -200,15 +228,14 @@ __global__ void __launch_bounds__(kRsWarps * 32, 1)
             // hold a row start; lane 0 continues the previous chunk's row
             T sc = run;
             if (lane == 0 && !seen) sc += carry;
-            bool r = seen;
+            // bit l of cont: the d lanes up to l all go on from the lane before
+            uint32_t cont = ~heads & ~1u;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
+                if (cont == 0) break;  // no row reaches d lanes further
                 const T su = __shfl_up_sync(kFull, sc, d);
-                const bool ru = __shfl_up_sync(kFull, (int)r, d) != 0;
-                if (lane >= d) {
-                    if (!r) sc += su;
-                    r = r || ru;
-                }
+                if ((cont >> lane) & 1u) sc += su;
+                cont &= cont << d;
             }
             T cin = __shfl_up_sync(kFull, sc, 1);
             if (lane == 0) cin = carry;
@@ -675,28 +702,40 @@ __global__ void cb_balanced_values_kernel(const BalancedDev b, const uint8_t *__
 
 }  // namespace
 
-template <typename T, bool UNIT>
+template <typename T, bool UNIT, bool MAP>
 const void *rowseg_fn() {
-    return reinterpret_cast<const void *>(cb_rowseg_kernel<T, UNIT>);
+    return reinterpret_cast<const void *>(cb_rowseg_kernel<T, UNIT, MAP>);
+}
+
+template <typename T, bool UNIT, bool MAP>
+cudaError_t launch_rowseg_m(const DevLayout &d, const void *x, void *y, size_t smem,
+                            cudaStream_t stream) {
+    const void *fn = rowseg_fn<T, UNIT, MAP>();
+    cudaError_t e = dev_enable_smem(fn, smem);
+    if (e != cudaSuccess) return e;
+    // the carveout: what the window leaves is L1 for the other gathers.  In
+    // powers of two, so that plans of about one window size share a setting
+    // (a change costs the host a call)
+    size_t keep = size_t(16) << 10;
+    while (keep < smem) keep *= 2;
+    dev_resident_l1(fn, kRsWarps * 32, keep);
+    // the grid the segments and windows were assigned for
+    cb_rowseg_kernel<T, UNIT, MAP><<<(unsigned)d.rs.G, kRsWarps * 32, smem, stream>>>(
+        d.rs, static_cast<const T *>(x), static_cast<T *>(y));
+    return cudaSuccess;
 }
 
 template <typename T, bool UNIT>
 cudaError_t launch_rowseg_t(const DevLayout &d, const void *x, void *y, size_t smem,
                             cudaStream_t stream) {
-    const void *fn = rowseg_fn<T, UNIT>();
-    cudaError_t e = dev_enable_smem(fn, smem);
-    if (e != cudaSuccess) return e;
-    dev_resident_l1(fn, kRsWarps * 32, smem);  // sets the carveout
-    // the grid the segments and windows were assigned for
-    cb_rowseg_kernel<T, UNIT><<<(unsigned)d.rs.G, kRsWarps * 32, smem, stream>>>(
-        d.rs, static_cast<const T *>(x), static_cast<T *>(y));
-    return cudaSuccess;
+    return d.rs.rowmap ? launch_rowseg_m<T, UNIT, true>(d, x, y, smem, stream)
+                       : launch_rowseg_m<T, UNIT, false>(d, x, y, smem, stream);
 }
 
 int64_t rowseg_warps(int f32) {
     // the x window in shared memory; the carveout leaves the rest of the
     // unified L1/shared memory to the L1 (the other x gathers)
-    const void *fn = f32 ? rowseg_fn<float, false>() : rowseg_fn<double, false>();
+    const void *fn = f32 ? rowseg_fn<float, false, true>() : rowseg_fn<double, false, true>();
     if (dev_enable_smem(fn, (size_t)kRsWindowBytes) != cudaSuccess) {
         cudaGetLastError();
         return 0;
@@ -706,7 +745,7 @@ int64_t rowseg_warps(int f32) {
 }
 
 cudaError_t launch_rowseg(const DevLayout &d, const void *x, void *y, cudaStream_t stream) {
-    if (!d.rs.chunks || d.rs.nseg <= 0 || d.rs.G <= 0 || !d.rs.wbase)
+    if (!d.rs.chunks || d.rs.nseg <= 0 || d.rs.G <= 0 || !d.rs.wbase || !d.rs.wlen)
         return cudaErrorInvalidValue;
     const size_t smem = (size_t)d.rs.W * (d.f32 ? 4 : 8);
     const cudaError_t e =
