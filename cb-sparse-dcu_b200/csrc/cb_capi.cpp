@@ -66,11 +66,13 @@ struct DevSide {
     int partial_nrhs = 0;
     int64_t *vsrc_ptr = nullptr;
     int32_t *vsrc = nullptr;
+    bool one_source = false;        // every stored value has one input: vsrc and
+                                    // val_off on the device are in payload order
     uint64_t *val_off = nullptr;
     int32_t *val_row = nullptr, *val_col = nullptr;
     int32_t *pat[4] = {};  // pattern row_ptr, col_idx, output_ptr, output_rows
     // row-segment stream (kernel 5): chunks, segment meta, spans, counters,
-    // partial slots, rowmap, empty rows, value positions, window bases, window lengths
+    // partial slots, rowmap, empty rows, value positions or entries' inputs, window bases, window lengths
     void *rs[10] = {};
     int64_t rs_bytes = 0;
     std::vector<int32_t> rs_cinfo;  // per chunk summaries (batches cut their own segments)
@@ -218,9 +220,31 @@ cbspmv_status upload_side(DevSide &s, cudaStream_t st) {
     CB_CUDA(upload_vec(L.blocks, (cb::BlockDesc **)&s.blocks, st), "upload blocks");
     CB_CUDA(upload_vec(L.payload, &s.payload, st), "upload payload");
     CB_CUDA(upload_vec(L.block_cols, &s.block_cols, st), "upload gather list");
-    CB_CUDA(upload_vec(L.vsrc_ptr, &s.vsrc_ptr, st), "upload value sources");
-    CB_CUDA(upload_vec(L.vsrc, &s.vsrc, st), "upload value sources");
-    CB_CUDA(upload_vec(L.val_off, &s.val_off, st), "upload value offsets");
+    s.one_source = !L.unit && (int64_t)L.vsrc.size() == L.nvals &&
+                   (int64_t)L.vsrc_ptr.size() == L.nvals + 1;
+    for (int64_t v = 0; s.one_source && v < L.nvals; ++v)
+        s.one_source = L.vsrc_ptr[(size_t)v] == v;
+    if (s.one_source) {  // sources and offsets in payload order (ValueSide)
+        const size_t vsz = L.f32 ? 4 : 8;
+        std::vector<int32_t> at(L.payload.size() / vsz, -1);
+        for (size_t v = 0; v < L.vsrc.size(); ++v) at[L.val_off[v] / vsz] = (int32_t)v;
+        std::vector<int32_t> src;
+        std::vector<uint64_t> off;
+        src.reserve(L.vsrc.size());
+        off.reserve(L.vsrc.size());
+        for (int32_t v : at)
+            if (v >= 0) {
+                src.push_back(L.vsrc[(size_t)v]);
+                off.push_back(L.val_off[(size_t)v]);
+            }
+        CB_CUDA(upload_vec(src, &s.vsrc, st), "upload value sources");
+        CB_CUDA(upload_vec(off, &s.val_off, st), "upload value offsets");
+        CB_CUDA(cudaStreamSynchronize(st), "upload value sources");
+    } else {
+        CB_CUDA(upload_vec(L.vsrc_ptr, &s.vsrc_ptr, st), "upload value sources");
+        CB_CUDA(upload_vec(L.vsrc, &s.vsrc, st), "upload value sources");
+        CB_CUDA(upload_vec(L.val_off, &s.val_off, st), "upload value offsets");
+    }
     CB_CUDA(upload_vec(L.val_row, &s.val_row, st), "upload value rows");
     CB_CUDA(upload_vec(L.val_col, &s.val_col, st), "upload value columns");
     // scratch: 4 scheduler words (next tile, warps done, error word, spare),
@@ -320,7 +344,16 @@ cbspmv_status upload_rowseg(DevSide &s, int kernel, cudaStream_t st) {
             "allocate row-segment slots");
     CB_CUDA(upload_vec(R.rowmap, (int32_t **)&s.rs[5], st), "upload row segments");
     CB_CUDA(upload_vec(R.empty, (int32_t **)&s.rs[6], st), "upload row segments");
-    CB_CUDA(upload_vec(R.vpos, (int32_t **)&s.rs[7], st), "upload row segments");
+    std::vector<int32_t> ssrc;  // per stream entry its input (ValueSide)
+    if (s.one_source && !R.vpos.empty()) {
+        ssrc.assign((size_t)R.nch * cb::rs_chunk_entries(), -1);
+        for (size_t v = 0; v < R.vpos.size(); ++v)
+            if (R.vpos[v] >= 0) ssrc[(size_t)R.vpos[v]] = s.lay.vsrc[v];
+        CB_CUDA(upload_vec(ssrc, (int32_t **)&s.rs[7], st), "upload row segments");
+        CB_CUDA(cudaStreamSynchronize(st), "upload row segments");
+    } else {
+        CB_CUDA(upload_vec(R.vpos, (int32_t **)&s.rs[7], st), "upload row segments");
+    }
     CB_CUDA(upload_vec(R.wbase, (int32_t **)&s.rs[8], st), "upload row segments");
     CB_CUDA(upload_vec(R.wlen, (int32_t **)&s.rs[9], st), "upload row segments");
     cb::RowSegDev &d = s.d.rs;
@@ -336,7 +369,10 @@ cbspmv_status upload_rowseg(DevSide &s, int kernel, cudaStream_t st) {
     d.rowmap = R.rowmap.empty() ? nullptr : static_cast<const int32_t *>(s.rs[5]);
     d.empty = static_cast<const int32_t *>(s.rs[6]);
     d.nempty = (int32_t)R.empty.size();
-    d.vpos = static_cast<const int32_t *>(s.rs[7]);
+    if (ssrc.empty())
+        d.vpos = static_cast<const int32_t *>(s.rs[7]);
+    else
+        d.ssrc = static_cast<const int4 *>(s.rs[7]);
     d.G = R.G;
     // (at least one value: the launch asks for the longest window in use)
     d.W = std::max<int32_t>(1, *std::max_element(R.wlen.begin(), R.wlen.end()));
@@ -1152,16 +1188,24 @@ cbspmv_status cbspmv_set_values(cbspmv_plan *p, const void *input_values,
                     "this plan stores no values (every value was 1); build it with "
                     "keep_values = 1 to change them");
     cudaStream_t st = (cudaStream_t)stream;
-    DevSide *sides[2] = {&p->A, p->has_t ? &p->AT : nullptr};
-    for (DevSide *s : sides) {
-        if (!s) continue;
-        CB_CUDA(cb::launch_set_values(s->lay.f32, s->lay.nvals, s->vsrc_ptr, s->vsrc,
-                                      s->val_off, input_values, s->payload, st),
-                "set_values launch");
-        CB_CUDA(cb::launch_rowseg_values(s->d, s->lay.nvals, s->val_off, st),
-                "set_values launch");
-        CB_CUDA(cb::launch_balanced_values(s->d, st), "set_values launch");
-    }
+    auto side = [](const DevSide &s) {
+        cb::ValueSide v;
+        v.nvals = s.lay.nvals;
+        v.ptr = s.one_source ? nullptr : s.vsrc_ptr;
+        v.src = s.vsrc;
+        v.off = s.val_off;
+        v.payload = s.payload;
+        v.chunks = s.d.rs.vpos || s.d.rs.ssrc ? const_cast<uint8_t *>(s.d.rs.chunks) : nullptr;
+        v.vpos = s.d.rs.vpos;
+        v.ssrc = s.d.rs.ssrc;
+        v.nquads = (int64_t)s.d.rs.nch * (cb::rs_chunk_entries() / 4);
+        return v;
+    };
+    CB_CUDA(cb::launch_set_values(p->A.lay.f32, side(p->A),
+                                  p->has_t ? side(p->AT) : cb::ValueSide(), input_values, st),
+            "set_values launch");
+    CB_CUDA(cb::launch_balanced_values(p->A.d, st), "set_values launch");
+    if (p->has_t) CB_CUDA(cb::launch_balanced_values(p->AT.d, st), "set_values launch");
     return CBSPMV_OK;
 }
 

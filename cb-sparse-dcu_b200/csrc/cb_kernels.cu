@@ -36,6 +36,7 @@
 
 #include "cb_device.cuh"
 #include "cb_kernels.hpp"
+#include "cb_rowseg.hpp"
 
 namespace cb {
 namespace {
@@ -589,17 +590,80 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// Value v of a stream entry: its address in the chunks.
 template <typename T>
-__global__ void cb_set_values_kernel(int64_t nvals, const int64_t *__restrict__ ptr,
-                                     const int32_t *__restrict__ src,
-                                     const uint64_t *__restrict__ off,
-                                     const T *__restrict__ in,
-                                     uint8_t *__restrict__ payload) {
-    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= nvals) return;
-    T s = T(0);
-    for (int64_t z = ptr[v]; z < ptr[v + 1]; ++z) s += in[src[z]];
-    *reinterpret_cast<T *>(payload + off[v]) = s;
+__device__ __forceinline__ T *stream_value(uint8_t *chunks, int32_t e) {
+    constexpr int32_t C = 32 * kRsK, NV = 16 / (int32_t)sizeof(T);
+    constexpr int64_t CB = C * (4 + (int64_t)sizeof(T));
+    const int32_t c = e / C, i = e % C, l = i / kRsK, j = i % kRsK;
+    return reinterpret_cast<T *>(chunks + c * CB + 4 * C) + (j / NV) * 32 * NV + l * NV + j % NV;
+}
+
+// New values into the tile payload and the row-segment stream of both sides
+// in one launch: blocks [0, b0) take side a's values, [b0, b1) its stream
+// quads, [b1, b2) side t's values, the rest its quads.  Bound by the 32-byte
+// sectors that the reads and stores touch, so each destination is written in
+// its own order, where the stores are whole sectors (16 bytes a thread in the
+// stream); the sources of A's entries lie within a block row (L1), those of
+// A^T's are scattered, one sector each.  kSetU values a thread keep that many
+// reads in flight.
+constexpr int kSetU = 4;
+template <typename T>
+__global__ void __launch_bounds__(256)
+    cb_set_values_kernel(const ValueSide a, const ValueSide t, int64_t b0, int64_t b1,
+                         int64_t b2, const T *__restrict__ in) {
+    const int64_t b = blockIdx.x;
+    const ValueSide d = b < b1 ? a : t;
+    const bool quads = (b >= b0 && b < b1) || b >= b2;
+    const int64_t base = (b < b0 ? b : b < b1 ? b - b0 : b < b2 ? b - b1 : b - b2) * 256;
+    if (quads) {
+        const int64_t q = base + threadIdx.x;
+        if (q >= d.nquads) return;
+        const int4 z4 = __ldg(&d.ssrc[q]);
+        const int32_t z[4] = {z4.x, z4.y, z4.z, z4.w};
+        T v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = z[j] >= 0 ? T(0) + __ldg(&in[z[j]]) : T(0);
+        if constexpr (sizeof(T) == 4) {
+            *reinterpret_cast<float4 *>(stream_value<T>(d.chunks, (int32_t)(4 * q))) =
+                make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+            *reinterpret_cast<double2 *>(stream_value<T>(d.chunks, (int32_t)(4 * q))) =
+                make_double2(v[0], v[1]);
+            *reinterpret_cast<double2 *>(stream_value<T>(d.chunks, (int32_t)(4 * q + 2))) =
+                make_double2(v[2], v[3]);
+        }
+        return;
+    }
+    const int64_t v0 = base * kSetU + threadIdx.x;
+    if (!d.ptr) {  // one input per value
+        int32_t z[kSetU];
+        T s[kSetU];
+#pragma unroll
+        for (int u = 0; u < kSetU; ++u) {
+            const int64_t v = v0 + 256 * u;
+            z[u] = v < d.nvals ? __ldg(&d.src[v]) : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < kSetU; ++u)
+            s[u] = v0 + 256 * u < d.nvals ? T(0) + __ldg(&in[z[u]]) : T(0);
+#pragma unroll
+        for (int u = 0; u < kSetU; ++u) {
+            const int64_t v = v0 + 256 * u;
+            if (v < d.nvals) *reinterpret_cast<T *>(d.payload + __ldg(&d.off[v])) = s[u];
+        }
+        return;
+    }
+    for (int u = 0; u < kSetU; ++u) {  // several inputs in some value
+        const int64_t v = v0 + 256 * u;
+        if (v >= d.nvals) return;
+        T s = T(0);
+        for (int64_t z = __ldg(&d.ptr[v]), z1 = __ldg(&d.ptr[v + 1]); z < z1; ++z)
+            s += __ldg(&in[__ldg(&d.src[z])]);
+        *reinterpret_cast<T *>(d.payload + __ldg(&d.off[v])) = s;
+        // (no entry: a DENSE slot outside the valid rows and columns)
+        if (d.chunks && __ldg(&d.vpos[v]) >= 0) *stream_value<T>(d.chunks, __ldg(&d.vpos[v])) = s;
+    }
 }
 
 // LP lanes per value slot (a power of two): lane `sub` of a slot takes the
@@ -1004,18 +1068,19 @@ cudaError_t launch_spmv_fixed_scratch(const DevLayout &d, int64_t gb_m, int64_t 
     return launch_spmv(f, x, y, nrhs, ldx, ldy, stream);
 }
 
-cudaError_t launch_set_values(int f32, int64_t nvals, const int64_t *vsrc_ptr,
-                              const int32_t *vsrc, const uint64_t *val_off,
-                              const void *in, uint8_t *payload,
+cudaError_t launch_set_values(int f32, const ValueSide &a, const ValueSide &t, const void *in,
                               cudaStream_t stream) {
-    if (nvals == 0) return cudaSuccess;
-    const unsigned grid = (unsigned)((nvals + 255) / 256);
+    constexpr int64_t per = 256 * kSetU;
+    auto vb = [&](const ValueSide &s) { return (s.nvals + per - 1) / per; };
+    auto qb = [](const ValueSide &s) { return s.ssrc ? (s.nquads + 255) / 256 : int64_t(0); };
+    const int64_t b0 = vb(a), b1 = b0 + qb(a), b2 = b1 + vb(t), b3 = b2 + qb(t);
+    if (b3 == 0) return cudaSuccess;
     if (f32)
-        cb_set_values_kernel<float><<<grid, 256, 0, stream>>>(
-            nvals, vsrc_ptr, vsrc, val_off, static_cast<const float *>(in), payload);
+        cb_set_values_kernel<float><<<(unsigned)b3, 256, 0, stream>>>(
+            a, t, b0, b1, b2, static_cast<const float *>(in));
     else
-        cb_set_values_kernel<double><<<grid, 256, 0, stream>>>(
-            nvals, vsrc_ptr, vsrc, val_off, static_cast<const double *>(in), payload);
+        cb_set_values_kernel<double><<<(unsigned)b3, 256, 0, stream>>>(
+            a, t, b0, b1, b2, static_cast<const double *>(in));
     note_launch();
     return cudaGetLastError();
 }

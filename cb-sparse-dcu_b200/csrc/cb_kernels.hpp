@@ -20,7 +20,10 @@ struct RowSegDev {
     const int32_t *rowmap = nullptr;  // ordinal -> row, NULL when every row is non-empty
     const int32_t *empty = nullptr;   // rows without stored entries
     int32_t nempty = 0;
-    const int32_t *vpos = nullptr;    // per stored value: its stream entry
+    // for value updates (ValueSide): per stored value its stream entry, or,
+    // when every stored value has one input, per stream entry its input
+    const int32_t *vpos = nullptr;
+    const int4 *ssrc = nullptr;
     int32_t G = 0, W = 0;             // CTAs of every launch; longest window (values)
     const int32_t *wbase = nullptr;   // per CTA: first column of its x window
     const int32_t *wlen = nullptr;    // per CTA: columns of its x window
@@ -164,8 +167,7 @@ cudaError_t launch_pattern(const DevLayout &d, const void *x, void *y, cudaStrea
 
 // Row-segment stream (cb_rowseg_kernels.cu): warps of one launch on the current
 // device (one CTA of kRsWarps warps per SM; 0 when the kernel cannot run);
-// y = A x over d.rs; the stream's values refreshed from the tile payload
-// (after the payload's values changed).
+// y = A x over d.rs.
 int64_t rowseg_warps(int f32);
 cudaError_t launch_rowseg(const DevLayout &d, const void *x, void *y, cudaStream_t stream);
 // Y = A X over d.rs for nrhs right-hand sides (row-major, leading dims ldx,
@@ -173,8 +175,6 @@ cudaError_t launch_rowseg(const DevLayout &d, const void *x, void *y, cudaStream
 constexpr int kRsSlotValues = 16;
 cudaError_t launch_rowseg_mrhs(const DevLayout &d, const void *x, void *y, int nrhs,
                                int64_t ldx, int64_t ldy, cudaStream_t stream);
-cudaError_t launch_rowseg_values(const DevLayout &d, int64_t nvals, const uint64_t *val_off,
-                                 cudaStream_t stream);
 
 // The fused adjoint over a transposed plan's stream d.rs (values stored):
 // gx = A^T g (n x nrhs, the stream's rows) and, per stream entry e of row j
@@ -232,10 +232,26 @@ cudaError_t launch_spmv_fixed_scratch(const DevLayout &d, int64_t gb_m, int64_t 
                                       const void *x, void *y, int nrhs, int64_t ldx,
                                       int64_t ldy, cudaStream_t stream);
 
-// payload value v = sum of in[vsrc[z]] for z in [vsrc_ptr[v], vsrc_ptr[v+1])
-cudaError_t launch_set_values(int f32, int64_t nvals, const int64_t *vsrc_ptr,
-                              const int32_t *vsrc, const uint64_t *val_off,
-                              const void *in, uint8_t *payload,
+// One side of a value update: stored value v = sum of in[src[z]] for z in
+// [ptr[v], ptr[v+1]), written at payload + off[v] and, when chunks is not NULL
+// and vpos[v] >= 0, as the value of row-segment stream entry vpos[v].
+// ptr NULL (every stored value has one input): stored value v = in[src[v]] at
+// payload + off[v], v in payload order, and the stream, when chunks is not
+// NULL, from its own sources: entry e = in[ssrc[e]] (0 for ssrc[e] < 0),
+// 4 entries per int4, nquads of them.
+struct ValueSide {
+    int64_t nvals = 0;
+    const int64_t *ptr = nullptr;
+    const int32_t *src = nullptr;
+    const uint64_t *off = nullptr;
+    uint8_t *payload = nullptr;
+    uint8_t *chunks = nullptr;
+    const int32_t *vpos = nullptr;
+    const int4 *ssrc = nullptr;
+    int64_t nquads = 0;
+};
+// Both sides (nvals 0: absent) of a plan in one launch.
+cudaError_t launch_set_values(int f32, const ValueSide &a, const ValueSide &t, const void *in,
                               cudaStream_t stream);
 
 // gvals[v] = sum_j g[row_v * ldg + j] * x[col_v * ldx + j] (0 when the slot

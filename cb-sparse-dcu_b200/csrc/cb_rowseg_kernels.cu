@@ -7,7 +7,7 @@
 //   * cb_rowseg_batch_kernel every matrix of a batch in one launch;
 //   * cb_balanced_kernel     plans built with row_owned = 0: the reference's
 //                            block order, atomics into y;
-//   * value refreshes after cbspmv_set_values.
+//   * the balanced stream's value refresh after cbspmv_set_values.
 //
 // One right-hand side: one CTA of 32 warps per SM.  Per chunk a lane
 //   * holds the NEXT chunk's words and values in registers, loaded with
@@ -621,26 +621,6 @@ __global__ void __launch_bounds__(kRsBatchWarps * 32, 1)
     }
 }
 
-// Stream values refreshed from the tile payload: chunks[value of entry
-// vpos[v]] = payload value v.
-template <typename T>
-__global__ void cb_rowseg_values_kernel(const RowSegDev rs, const uint8_t *__restrict__ payload,
-                                        const uint64_t *__restrict__ val_off, int64_t nvals) {
-    constexpr int64_t C = 32 * kRsK, NV = 16 / sizeof(T);
-    constexpr int64_t CB = C * (4 + (int64_t)sizeof(T));
-    uint8_t *chunks = const_cast<uint8_t *>(rs.chunks);
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < nvals;
-         v += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t e = __ldg(&rs.vpos[v]);
-        if (e < 0) continue;  // a DENSE slot outside the valid rows and columns
-        const int64_t c = e / C, i = e % C, l = i / kRsK, j = i % kRsK;
-        const int64_t pos = (j / NV) * 32 * NV + l * NV + j % NV;
-        *reinterpret_cast<T *>(chunks + c * CB + 4 * C + pos * (int64_t)sizeof(T)) =
-            *reinterpret_cast<const T *>(payload + __ldg(&val_off[v]));
-    }
-}
-
-
 // The balanced schedule (plans built with row_owned = 0): warps take whole
 // groups (the reference's CTAs of waves_per_block blocks, balanced by its
 // permutation), each lane a quad of 4 entries at a time; a run of one row
@@ -916,20 +896,6 @@ cudaError_t launch_rowseg_batch(int f32, const RsBatchMat *mats, const int4 *seg
         cb_rowseg_batch_kernel<double><<<grid, kRsBatchWarps * 32, 0, stream>>>(
             mats, segs, meta, nseg, sched, empty, nempty, spans, counters,
             static_cast<double *>(part));
-    note_launch();
-    return cudaGetLastError();
-}
-
-cudaError_t launch_rowseg_values(const DevLayout &d, int64_t nvals, const uint64_t *val_off,
-                                 cudaStream_t stream) {
-    if (!d.rs.chunks || !d.rs.vpos || nvals <= 0) return cudaSuccess;
-    const unsigned grid =
-        (unsigned)std::min<int64_t>((nvals + 255) / 256, (int64_t)dev_sms() * 16);
-    if (d.f32)
-        cb_rowseg_values_kernel<float><<<grid, 256, 0, stream>>>(d.rs, d.payload, val_off, nvals);
-    else
-        cb_rowseg_values_kernel<double><<<grid, 256, 0, stream>>>(d.rs, d.payload, val_off,
-                                                                  nvals);
     note_launch();
     return cudaGetLastError();
 }
