@@ -112,6 +112,8 @@ def _load():
                                             _I64, _P]),
         "cbspmv_adjoint": (ctypes.c_int, [_P, _P, _P, _P, _P, ctypes.c_int, _I64, _I64,
                                           _I64, _P]),
+        "cbspmv_adjoint_input": (ctypes.c_int, [_P, _P, _P, _P, _P, ctypes.c_int, _I64, _I64,
+                                          _I64, _P]),
         "cbspmv_num_values": (_I64, [_P]),
         "cbspmv_adjoint_fused": (ctypes.c_int, [_P, _P, _P, _P, _P, ctypes.c_int, _I64, _I64,
                                                 _I64, _P]),
@@ -429,6 +431,31 @@ class Plan:
                                    _dptr(gvals) if gvals is not None else None,
                                    k, k, k, k, _stream(stream)))
         return gx, gvals
+
+    def adjoint_input(self, g, x, gx=None, gin=None, want_gx=True, want_gin=True,
+                      stream=None):
+        """``adjoint`` with the value gradient in input order (the caller's
+        nonzeros): returns (gx, gin), None for an output not wanted.  The
+        first call uploads the nonzeros' rows and columns."""
+        import torch
+        self.upload(stream)
+        self._check_dev(g, x)
+        k = 1 if g.dim() == 1 else g.shape[1]
+        if want_gx and gx is None:
+            gx = torch.empty((self.n,) if g.dim() == 1 else (self.n, k),
+                             dtype=g.dtype, device=g.device)
+        if want_gin and gin is None:
+            gin = torch.empty(self.nnz, dtype=g.dtype, device=g.device)
+        gx = gx if want_gx else None
+        gin = gin if want_gin else None
+        for t in (gx, gin):
+            if t is not None:
+                self._check_dev(t)
+        _check(_lib.cbspmv_adjoint_input(self._h, _dptr(g), _dptr(x),
+                                         _dptr(gx) if gx is not None else None,
+                                         _dptr(gin) if gin is not None else None,
+                                         k, k, k, k, _stream(stream)))
+        return gx, gin
 
     def adjoint_fused(self, g, x, gx=None, gvals_t=None, stream=None):
         """(A^T g, value gradient) in one kernel launch on the transposed

@@ -6,12 +6,12 @@ caller's COO order) and X is (n,) or (n, k).  Backward:
 * dL/dX    = A^T dL/dY, on the plan's transposed CB layout (build the plan
   with ``want_transpose=1``);
 * dL/dvals = for each input nonzero k, dL/dY[row_k, :] . X[col_k, :],
-  computed per stored value of A (``adjoint``: the value-gradient kernel on
-  a second stream beside A^T dL/dY, the faster of the library's two adjoint
-  forms on the stream layouts) and gathered back to input order through
-  ``input_slots`` -- every input is summed into exactly one stored value, so
-  that value's gradient is the input's gradient.  ``adjoint_fused`` (one
-  launch, gradient gathered through ``grad_positions_t``) computes the same.
+  computed in input order (``adjoint_input``: the value-gradient kernel over
+  the input nonzeros' rows and columns, on a second stream beside
+  A^T dL/dY) -- every input is summed into exactly one stored value, so that
+  value's gradient is the input's gradient.  ``adjoint`` (per stored value,
+  gathered through ``input_slots``) and ``adjoint_fused`` (one launch,
+  gathered through ``grad_positions_t``) compute the same.
 
 Build the plan with ``keep_values=1`` when its initial values may all be 1:
 a unit-valued plan stores no values and cannot take new ones.
@@ -40,14 +40,7 @@ class CBSpMVFunction(torch.autograd.Function):
             return None, None, None
         # both in one call: the value gradient overlaps A^T g on a second
         # stream
-        gx, gslots = plan.adjoint(gy, x.contiguous(), want_gx=want_gx, want_gvals=want_v)
-        gvals = None
-        if want_v:
-            slots = getattr(plan, "_slots_dev", None)
-            if slots is None or slots.device != gy.device:
-                slots = torch.from_numpy(plan.input_slots()).to(gy.device)
-                plan._slots_dev = slots
-            gvals = gslots[slots]
+        gx, gvals = plan.adjoint_input(gy, x.contiguous(), want_gx=want_gx, want_gin=want_v)
         return gvals, gx, None
 
 

@@ -11,6 +11,7 @@
 #include <cstring>
 #include <future>
 #include <new>
+#include <mutex>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -162,6 +163,10 @@ struct cbspmv_plan {
     // cbspmv_adjoint: the value gradient's stream and its fork/join events
     cudaStream_t adj = nullptr;
     cudaEvent_t adj_fork = nullptr, adj_join = nullptr;
+    // cbspmv_adjoint_input: the input nonzeros' rows and columns
+    std::mutex in_mu;
+    bool in_ready = false;
+    int32_t *in_row = nullptr, *in_col = nullptr;
     // error words of A's and A^T's launches (host-mapped pinned memory, so the
     // host reads them without a copy): set by a kernel whose bounded wait gave
     // up; herr is the host view, derr the device view
@@ -176,6 +181,8 @@ struct cbspmv_plan {
         AT.release();
         if (hx) cudaFree(hx);
         if (hy) cudaFree(hy);
+        if (in_row) cudaFree(in_row);
+        if (in_col) cudaFree(in_col);
         if (herr) cudaFreeHost(herr);
     }
 };
@@ -1072,16 +1079,34 @@ cbspmv_status cbspmv_grad_vals(cbspmv_plan *p, const void *g, const void *x,
     return CBSPMV_OK;
 }
 
-cbspmv_status cbspmv_adjoint(cbspmv_plan *p, const void *g, const void *x, void *gx,
-                             void *gvals, int nrhs, int64_t ldg, int64_t ldx, int64_t ldgx,
-                             void *stream) {
-    if (!p) return fail(CBSPMV_ERR_INVALID, "null plan");
-    if (!gx && !gvals) return fail(CBSPMV_ERR_INVALID, "neither gx nor gvals given");
-    if (gx && !p->has_t) return fail(CBSPMV_ERR_STATE, "plan built without want_transpose");
-    if (!gx) return cbspmv_grad_vals(p, g, x, gvals, nrhs, ldg, ldx, stream);
-    if (!gvals) return cbspmv_spmv_t(p, g, gx, nrhs, ldg, ldgx, stream);
-    if (cbspmv_status rc = refuse_spmv_only(p)) return rc;
-    if (!p->uploaded) return fail(CBSPMV_ERR_STATE, "plan not uploaded");
+}  // extern "C"
+
+namespace {
+// The rows and columns of the input nonzeros on the device (the caller's
+// order), uploaded by the first call that needs them.
+cbspmv_status ensure_input_coords(cbspmv_plan *p, cudaStream_t st) {
+    std::lock_guard<std::mutex> lock(p->in_mu);
+    if (p->in_ready) return CBSPMV_OK;
+    const cb::DeviceLayout &L = p->A.lay;
+    const size_t nnz = (size_t)p->host.nnz;
+    std::vector<int32_t> row(nnz), col(nnz);
+    for (size_t i = 0; i < nnz; ++i) {
+        row[i] = L.val_row[(size_t)L.input_slot[i]];
+        col[i] = L.val_col[(size_t)L.input_slot[i]];
+    }
+    if (!p->in_row) CB_CUDA(upload_vec(row, &p->in_row, st), "upload input coordinates");
+    if (!p->in_col) CB_CUDA(upload_vec(col, &p->in_col, st), "upload input coordinates");
+    CB_CUDA(cudaStreamSynchronize(st), "upload input coordinates");
+    p->in_ready = true;
+    return CBSPMV_OK;
+}
+
+// A^T g on `stream` and the gradient of the values at (row[v], col[v]),
+// v < nvals, on the plan's second stream.
+cbspmv_status adjoint_pair(cbspmv_plan *p, int64_t nvals, const int32_t *row,
+                           const int32_t *col, const void *g, const void *x, void *gx,
+                           void *gvals, int nrhs, int64_t ldg, int64_t ldx, int64_t ldgx,
+                           void *stream) {
     if (nrhs < 1) return fail(CBSPMV_ERR_INVALID, "nrhs must be >= 1");
     const int64_t lg = ldg ? ldg : nrhs, lx = ldx ? ldx : nrhs;
     if (lg < nrhs || lx < nrhs)
@@ -1098,15 +1123,58 @@ cbspmv_status cbspmv_adjoint(cbspmv_plan *p, const void *g, const void *x, void 
     cudaStream_t st = (cudaStream_t)stream;
     CB_CUDA(cudaEventRecord(p->adj_fork, st), "adjoint fork");
     CB_CUDA(cudaStreamWaitEvent(p->adj, p->adj_fork, 0), "adjoint fork");
-    DevSide &s = p->A;
-    CB_CUDA(cb::launch_grad_vals(s.lay.f32, s.lay.nvals, s.val_row, s.val_col, g, lg, x, lx,
-                                 nrhs, gvals, p->adj),
+    CB_CUDA(cb::launch_grad_vals(p->A.lay.f32, nvals, row, col, g, lg, x, lx, nrhs, gvals,
+                                 p->adj),
             "grad_vals launch");
     const cbspmv_status rc = run_side(p, p->AT, g, gx, nrhs, lg, ldgx, st);
     // join even when A^T g failed, so no work is left unordered on `stream`
     CB_CUDA(cudaEventRecord(p->adj_join, p->adj), "adjoint join");
     CB_CUDA(cudaStreamWaitEvent(st, p->adj_join, 0), "adjoint join");
     return rc;
+}
+}  // namespace
+
+extern "C" {
+
+cbspmv_status cbspmv_adjoint(cbspmv_plan *p, const void *g, const void *x, void *gx,
+                             void *gvals, int nrhs, int64_t ldg, int64_t ldx, int64_t ldgx,
+                             void *stream) {
+    if (!p) return fail(CBSPMV_ERR_INVALID, "null plan");
+    if (!gx && !gvals) return fail(CBSPMV_ERR_INVALID, "neither gx nor gvals given");
+    if (gx && !p->has_t) return fail(CBSPMV_ERR_STATE, "plan built without want_transpose");
+    if (!gx) return cbspmv_grad_vals(p, g, x, gvals, nrhs, ldg, ldx, stream);
+    if (!gvals) return cbspmv_spmv_t(p, g, gx, nrhs, ldg, ldgx, stream);
+    if (cbspmv_status rc = refuse_spmv_only(p)) return rc;
+    if (!p->uploaded) return fail(CBSPMV_ERR_STATE, "plan not uploaded");
+    return adjoint_pair(p, p->A.lay.nvals, p->A.val_row, p->A.val_col, g, x, gx, gvals, nrhs, ldg,
+                        ldx, ldgx, stream);
+}
+
+cbspmv_status cbspmv_adjoint_input(cbspmv_plan *p, const void *g, const void *x, void *gx,
+                                   void *gin, int nrhs, int64_t ldg, int64_t ldx, int64_t ldgx,
+                                   void *stream) {
+    if (!p) return fail(CBSPMV_ERR_INVALID, "null plan");
+    if (!gx && !gin) return fail(CBSPMV_ERR_INVALID, "neither gx nor gin given");
+    if (gx && !p->has_t) return fail(CBSPMV_ERR_STATE, "plan built without want_transpose");
+    if (!gin) return cbspmv_spmv_t(p, g, gx, nrhs, ldg, ldgx, stream);
+    if (cbspmv_status rc = refuse_spmv_only(p)) return rc;
+    if (!p->uploaded) return fail(CBSPMV_ERR_STATE, "plan not uploaded");
+    if (nrhs < 1) return fail(CBSPMV_ERR_INVALID, "nrhs must be >= 1");
+    int dev = -1;
+    cudaGetDevice(&dev);
+    if (dev != p->device) return fail(CBSPMV_ERR_STATE, "plan was uploaded to another device");
+    const cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (cbspmv_status rc = ensure_input_coords(p, st)) return rc;
+    if (gx)
+        return adjoint_pair(p, p->host.nnz, p->in_row, p->in_col, g, x, gx, gin, nrhs, ldg, ldx,
+                            ldgx, stream);
+    const int64_t lg = ldg ? ldg : nrhs, lx = ldx ? ldx : nrhs;
+    if (lg < nrhs || lx < nrhs)
+        return fail(CBSPMV_ERR_INVALID, "leading dimension smaller than nrhs");
+    CB_CUDA(cb::launch_grad_vals(p->A.lay.f32, p->host.nnz, p->in_row, p->in_col, g, lg, x, lx,
+                                 nrhs, gin, st),
+            "grad_vals launch");
+    return CBSPMV_OK;
 }
 
 namespace {

@@ -249,6 +249,15 @@ cbspmv_status cbspmv_adjoint(cbspmv_plan *plan, const void *g, const void *x,
                              void *gx, void *gvals, int nrhs, int64_t ldg,
                              int64_t ldx, int64_t ldgx, void *stream);
 
+/* cbspmv_adjoint with the value gradient in the caller's input order: gin[k]
+ * is the gradient of input nonzero k (every input is summed into exactly one
+ * stored value, so it is that value's gradient).  The first call uploads the
+ * input nonzeros' rows and columns (and waits for it), so make it before
+ * capturing one. */
+cbspmv_status cbspmv_adjoint_input(cbspmv_plan *plan, const void *g, const void *x,
+                             void *gx, void *gin, int nrhs, int64_t ldg,
+                             int64_t ldx, int64_t ldgx, void *stream);
+
 /* The backward pass of Y = A X in ONE kernel launch on the transposed
  * layout (plans built with want_transpose and with stored values): gx = A^T g
  * and, from the same gathered rows of g, the value gradient of every stored

@@ -1,6 +1,7 @@
-"""Value updates (GPU): a plan given new values gives bit for bit what a plan
-built with them gives, from the stream and from the tiles, forward and
-transposed."""
+"""Value updates and gradients in input order (GPU): a plan given new values
+gives bit for bit what a plan built with them gives, from the stream and from
+the tiles, forward and transposed; the input-order gradient is the stored
+values' gradient, value for value."""
 import numpy as np
 import pytest
 
@@ -45,3 +46,24 @@ def test_new_values_as_if_built_with_them(cuda, kind, nnz, f32, kernel):
     g = torch.randn(coo.m, device=cuda, dtype=dt)
     assert torch.equal(p.spmv(x), q.spmv(x))
     assert torch.equal(p.spmv_t(g), q.spmv_t(g))
+
+
+@pytest.mark.parametrize("kind,nnz", [("random", 1), ("random", 1025), ("band", 1024),
+                                      ("dups", 2500)])
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("nrhs", [1, 3, 8])
+def test_adjoint_in_input_order(cuda, kind, nnz, f32, nrhs):
+    import torch
+    import cbspmv
+    coo, _ = _case(kind, nnz)
+    dt = torch.float32 if f32 else torch.float64
+    plan = cbspmv.Plan(coo, value_type=int(f32), want_transpose=1, keep_values=1)
+    shape = (nrhs,) if nrhs > 1 else ()
+    x = torch.randn((coo.n,) + shape, device=cuda, dtype=dt)
+    g = torch.randn((coo.m,) + shape, device=cuda, dtype=dt)
+    gx, gslots = plan.adjoint(g, x)
+    hx, gin = plan.adjoint_input(g, x)
+    slots = torch.from_numpy(plan.input_slots()).to(cuda)
+    assert torch.equal(gx, hx) and torch.equal(gslots[slots], gin)
+    none, only = plan.adjoint_input(g, x, want_gx=False)
+    assert none is None and torch.equal(only, gin)
