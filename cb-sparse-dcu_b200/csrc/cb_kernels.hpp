@@ -29,7 +29,6 @@ struct RowSegDev {
     const int32_t *wlen = nullptr;    // per CTA: columns of its x window
     int64_t n = 0;                    // columns (length of x)
     int unit = 0;                     // words only: every stored value is 1
-    int auto1 = 0;                    // the automatic choice for one right-hand side
 };
 
 // The balanced schedule's stream on the device (cb_rowseg.hpp,

@@ -16,12 +16,6 @@ bool rowseg_applies(const DeviceLayout &L) {
     return L.nvals > 0 && L.n <= kRsMaxCols && L.m < (int64_t(1) << 31);
 }
 
-bool rowseg_all_coo(const DeviceLayout &L) {
-    for (const BlockDesc &b : L.blocks)
-        if (meta_type(b.meta) != 0) return false;  // a CSR or DENSE block
-    return true;
-}
-
 void rowseg_cut(const std::vector<int32_t> &cinfo, const std::vector<int64_t> &cuts,
                 int64_t seg0, int32_t tag, std::vector<int32_t> &meta,
                 std::vector<int32_t> &spans) {

@@ -99,11 +99,8 @@ struct RowSegHost {
 
 // Whether the layout takes the row-segment stream: stored entries, columns
 // below 2^30, rows below 2^31 (CSR and DENSE blocks are expanded into
-// entries).  rowseg_all_coo: every block is a COO block (the automatic choice
-// for one right-hand side then takes the stream; otherwise the tile kernels,
-// which read CSR/DENSE blocks with fewer index bytes).
+// entries).
 bool rowseg_applies(const DeviceLayout &L);
-bool rowseg_all_coo(const DeviceLayout &L);
 
 // Segment meta and spans of the segmentation `cuts` (chunk boundaries,
 // increasing, cuts.front() == 0, cuts.back() == nch) of one stream from its
