@@ -73,8 +73,9 @@ struct DevSide {
     int32_t *val_row = nullptr, *val_col = nullptr;
     int32_t *pat[4] = {};  // pattern row_ptr, col_idx, output_ptr, output_rows
     // row-segment stream (kernel 5): chunks, segment meta, spans, counters,
-    // partial slots, rowmap, empty rows, value positions or entries' inputs, window bases, window lengths
-    void *rs[10] = {};
+    // partial slots, rowmap, empty rows, value positions or entries' inputs, window bases, window lengths,
+    // exchange words
+    void *rs[11] = {};
     int64_t rs_bytes = 0;
     std::vector<int32_t> rs_cinfo;  // per chunk summaries (batches cut their own segments)
     std::vector<int32_t> rs_empty;  // rows without entries
@@ -330,6 +331,22 @@ cbspmv_status upload_partition(DevSide &s, int kernel, cudaStream_t st) {
     return CBSPMV_OK;
 }
 
+// A segmentation for the device: kRsPair on the head and tail spans that cover
+// two segments, and empty exchange words for all spans (the kernels' kEmpty).
+std::vector<int32_t> device_meta(const std::vector<int32_t> &meta,
+                                 const std::vector<int32_t> &spans) {
+    std::vector<int32_t> out(meta);
+    for (size_t s = 0; s < out.size(); s += 4)
+        for (size_t k = s + 2; k < s + 4; ++k)
+            if (out[k] >= 0 && spans[4 * (size_t)out[k] + 1] == spans[4 * (size_t)out[k]] + 1)
+                out[k] |= cb::kRsPair;
+    return out;
+}
+std::vector<uint32_t> empty_words(size_t nspan, size_t vsz) {
+    return std::vector<uint32_t>(std::max<size_t>(1, nspan) * cb::kRsSlotValues * vsz / 4,
+                                 0xffffdeadu);
+}
+
 // The row-segment stream (kernel 5; the automatic choice), segmented for this
 // device's resident warps.
 cbspmv_status upload_rowseg(DevSide &s, int kernel, cudaStream_t st) {
@@ -342,7 +359,10 @@ cbspmv_status upload_rowseg(DevSide &s, int kernel, cudaStream_t st) {
     const size_t vsz = s.lay.f32 ? 4 : 8;
     const std::vector<int32_t> zeros(std::max<size_t>(1, R.spans.size() / 4), 0);
     CB_CUDA(upload_vec(R.chunks, (uint8_t **)&s.rs[0], st), "upload row segments");
-    CB_CUDA(upload_vec(R.meta, (int32_t **)&s.rs[1], st), "upload row segments");
+    const std::vector<int32_t> meta = device_meta(R.meta, R.spans);
+    const std::vector<uint32_t> words = empty_words(R.spans.size() / 4, vsz);
+    CB_CUDA(upload_vec(meta, (int32_t **)&s.rs[1], st), "upload row segments");
+    CB_CUDA(upload_vec(words, (uint32_t **)&s.rs[10], st), "upload row segments");
     if (!R.spans.empty())
         CB_CUDA(upload_vec(R.spans, (int32_t **)&s.rs[2], st), "upload row segments");
     CB_CUDA(upload_vec(zeros, (int32_t **)&s.rs[3], st), "upload row segments");
@@ -372,6 +392,7 @@ cbspmv_status upload_rowseg(DevSide &s, int kernel, cudaStream_t st) {
     d.spans = static_cast<const int4 *>(s.rs[2]);
     d.counters = static_cast<int32_t *>(s.rs[3]);
     d.part = s.rs[4];
+    d.xch = s.rs[10];
     d.rowmap = R.rowmap.empty() ? nullptr : static_cast<const int32_t *>(s.rs[5]);
     d.empty = static_cast<const int32_t *>(s.rs[6]);
     d.nempty = (int32_t)R.empty.size();
@@ -1492,7 +1513,7 @@ struct cbspmv_batch {
     // over the row-segment streams (every plan has one, nrhs <= 16): the
     // matrices' table, segments {matrix, first chunk, end chunk, -} in queue
     // order with their meta, scheduler words, empty rows {matrix, row}, the
-    // batch's spans, counters and partial slots
+    // batch's spans, counters, partial slots and exchange words
     bool rs_mode = false;
     std::vector<cb::RsBatchMat> rmats;
     cb::RsBatchMat *d_rmats = nullptr;
@@ -1500,7 +1521,7 @@ struct cbspmv_batch {
     int32_t *d_rcnt = nullptr, nrseg = 0;
     uint32_t *d_rsched = nullptr;   // 2 scheduler words (next segment, warps out)
     int2 *d_rempty = nullptr;
-    void *d_rpart = nullptr;
+    void *d_rpart = nullptr, *d_rxch = nullptr;
     int64_t rwarps = 0, nrempty = 0;
     ~cbspmv_batch() {
         for (cudaGraphExec_t &g : exec)
@@ -1512,7 +1533,7 @@ struct cbspmv_batch {
         for (void *p : {(void *)d_toff, (void *)d_ustart, (void *)d_uorder, (void *)d_sched,
                         (void *)d_views, (void *)d_rmats, (void *)d_rsegs, (void *)d_rmeta,
                         (void *)d_rspans, (void *)d_rsched, (void *)d_rcnt, (void *)d_rempty,
-                        d_rpart})
+                        d_rpart, d_rxch})
             if (p) cudaFree(p);
         if (herr) cudaFreeHost(herr);
     }
@@ -1609,7 +1630,8 @@ cbspmv_status batch_rowseg_setup(cbspmv_batch *b, const int *nrhs) {
     const size_t nseg = segs.size() / 4, nspan = spans.size() / 4;
     const size_t vsz = b->f32 ? 4 : 8;
     cudaError_t e = upload_raw(segs, (int32_t **)&b->d_rsegs);
-    if (e == cudaSuccess) e = upload_raw(meta, (int32_t **)&b->d_rmeta);
+    if (e == cudaSuccess) e = upload_raw(device_meta(meta, spans), (int32_t **)&b->d_rmeta);
+    if (e == cudaSuccess) e = upload_raw(empty_words(nspan, vsz), (uint32_t **)&b->d_rxch);
     if (e == cudaSuccess) e = upload_raw(spans, (int32_t **)&b->d_rspans);
     if (e == cudaSuccess) e = upload_raw(std::vector<uint32_t>(2, 0u), &b->d_rsched);
     if (e == cudaSuccess) e = upload_raw(std::vector<int32_t>(std::max<size_t>(1, nspan), 0),
@@ -1642,7 +1664,7 @@ cbspmv_status batch_one(cbspmv_batch *b, cudaStream_t st) {
     if (b->rs_mode) {
         const cudaError_t e = cb::launch_rowseg_batch(
             b->f32, b->d_rmats, b->d_rsegs, b->d_rmeta, b->nrseg, b->d_rsched, b->rwarps,
-            b->d_rempty, b->nrempty, b->d_rspans, b->d_rcnt, b->d_rpart, st);
+            b->d_rempty, b->nrempty, b->d_rspans, b->d_rcnt, b->d_rpart, b->d_rxch, st);
         return e == cudaSuccess ? CBSPMV_OK : cuda_fail(e, "batch launch");
     }
     const cudaError_t e = cb::launch_batch(b->bs, b->f32, b->d_views, (int)b->plans.size(),

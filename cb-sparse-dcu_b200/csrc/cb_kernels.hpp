@@ -8,15 +8,21 @@
 
 namespace cb {
 
+// In the device's segment meta: the span covers two segments, which meet in
+// its exchange words (kRsSlotValues a span).
+constexpr int32_t kRsPair = 1 << 30;
+
 // The row-segment stream on the device (layout in cb_rowseg.hpp); chunks is
 // NULL when the plan has none.
 struct RowSegDev {
     const uint8_t *chunks = nullptr;
     int32_t nch = 0, M = 0, nseg = 0, nord = 0;
     const int4 *meta = nullptr;       // per segment: ord0, starts_row, head span, tail span
+                                      // (with kRsPair: a span of two segments)
     const int4 *spans = nullptr;      // per span: first segment, last segment, ordinal, 0
     int32_t *counters = nullptr;      // per span, zero between launches
     void *part = nullptr;             // 2 * nseg partial sums
+    void *xch = nullptr;              // exchange words of the spans of two segments
     const int32_t *rowmap = nullptr;  // ordinal -> row, NULL when every row is non-empty
     const int32_t *empty = nullptr;   // rows without stored entries
     int32_t nempty = 0;
@@ -209,12 +215,13 @@ int64_t rowseg_batch_warps(int f32);
 // zero before the first launch; the kernel leaves them zero), with meta[]
 // ({ordinal before, starts a row, head span, tail span}); empty rows {matrix,
 // row} are zeroed first; spans {first segment, last segment, ordinal, -},
-// counters (zero) and partial slots (kRsSlotValues values, two per segment)
-// belong to the batch.
+// counters (zero), partial slots (kRsSlotValues values, two per segment) and
+// exchange words belong to the batch.
 cudaError_t launch_rowseg_batch(int f32, const RsBatchMat *mats, const int4 *segs,
                                 const int4 *meta, int32_t nseg, uint32_t *sched, int64_t nwarps,
                                 const int2 *empty, int64_t nempty, const int4 *spans,
-                                int32_t *counters, void *part, cudaStream_t stream);
+                                int32_t *counters, void *part, void *xch,
+                                cudaStream_t stream);
 
 // y = A x; x: n rows, y: m rows, row-major with leading dims for nrhs > 1.
 cudaError_t launch_spmv(const DevLayout &d, const void *x, void *y, int nrhs,
