@@ -194,16 +194,19 @@ def _np_ptr(a: np.ndarray):
 
 
 def _stream(stream):
+    """The stream's handle, an int.  The current stream is asked for by its
+    raw handle: a torch.cuda.Stream object made for each call cost more than
+    the rest of a small product's host work."""
     if stream is None:
         import torch
-        return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-    if isinstance(stream, int):
-        return ctypes.c_void_p(stream)
-    return ctypes.c_void_p(stream.cuda_stream)
+        if not torch.cuda.is_initialized():
+            torch.cuda.init()
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    return stream if isinstance(stream, int) else stream.cuda_stream
 
 
 def _dptr(t):
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 INT_EXPORTS = [
@@ -354,7 +357,8 @@ class Plan:
         if y is None:
             y = torch.empty((self.m,) if x.dim() == 1 else (self.m, k),
                             dtype=x.dtype, device=x.device)
-        self._check_dev(y)
+        else:
+            self._check_dev(y)
         _check(_lib.cbspmv_spmv(self._h, _dptr(x), _dptr(y), k, k, k,
                                 _stream(stream)))
         return y

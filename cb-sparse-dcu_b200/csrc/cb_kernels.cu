@@ -906,6 +906,8 @@ std::map<int, int> g_sms;                                    // device -> SMs
 std::map<std::pair<int, const void *>, size_t> g_smem;       // (device, kernel) -> enabled
 std::map<std::tuple<int, const void *, int, size_t>, int> g_resident;
 std::map<std::pair<int, const void *>, int> g_carve;        // carveout set + 1
+// resident blocks and carveout of dev_resident_l1
+std::map<std::tuple<int, const void *, int, size_t>, std::pair<int, int>> g_l1;
 std::atomic<uint32_t> g_wait_polls{0};                       // 0: kWaitLimit
 
 int current_device() {
@@ -951,21 +953,36 @@ int dev_resident(const void *fn, int threads, size_t smem) {
 }
 
 int dev_resident_l1(const void *fn, int threads, size_t smem) {
+    // the blocks and the carveout are worked out once per kernel and
+    // footprint: the attribute queries were most of a small launch's own host
+    // time
+    const int d = current_device();
+    const auto key = std::make_tuple(d, fn, threads, smem);
+    {
+        std::lock_guard<std::mutex> lock(g_facts_mu);
+        auto it = g_l1.find(key);
+        if (it != g_l1.end() && (it->second.second < 0 ||
+                                 g_carve[{d, fn}] == it->second.second + 1))
+            return it->second.first;
+    }
     // the occupancy query counts the carveout preference a previous launch
     // set for a smaller footprint, so take the register and thread limit
     // alone and the shared-memory limit from the largest carveout
     int r = dev_resident(fn, threads, 0);
-    const int d = current_device();
     int maxs = 0, reserved = 0;
     cudaDeviceGetAttribute(&maxs, cudaDevAttrMaxSharedMemoryPerMultiprocessor, d);
     cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, d);
-    if (maxs <= (int)kL1Keep) return r;
-    const size_t per = smem + (size_t)reserved;
-    const size_t cap = (size_t)maxs - kL1Keep;
-    r = std::min<int>(r, (int)((size_t)maxs / per));  // what fits at all
-    r = std::max(1, std::min<int>(r, (int)(cap / std::max<size_t>(per, 1))));
-    const int pct = (int)std::min<size_t>(100, (r * per * 100 + maxs - 1) / (size_t)maxs);
+    int pct = -1;  // no carveout to set
+    if (maxs > (int)kL1Keep) {
+        const size_t per = smem + (size_t)reserved;
+        const size_t cap = (size_t)maxs - kL1Keep;
+        r = std::min<int>(r, (int)((size_t)maxs / per));  // what fits at all
+        r = std::max(1, std::min<int>(r, (int)(cap / std::max<size_t>(per, 1))));
+        pct = (int)std::min<size_t>(100, (r * per * 100 + maxs - 1) / (size_t)maxs);
+    }
     std::lock_guard<std::mutex> lock(g_facts_mu);
+    g_l1[key] = {r, pct};
+    if (pct < 0) return r;
     int &have = g_carve[{d, fn}];
     if (have != pct + 1 &&
         cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, pct) ==
