@@ -606,7 +606,9 @@ __device__ __forceinline__ T *stream_value(uint8_t *chunks, int32_t e) {
 // its own order, where the stores are whole sectors (16 bytes a thread in the
 // stream); the sources of A's entries lie within a block row (L1), those of
 // A^T's are scattered, one sector each.  kSetU values a thread keep that many
-// reads in flight.
+// reads in flight.  At n = 100003, mean 24, FP32, with A^T: 30 us; in value
+// order with scattered stores 37, as a payload and a stream kernel a side 68;
+// A^T's payload read back from its stream, in a second launch, 31.
 constexpr int kSetU = 4;
 template <typename T>
 __global__ void __launch_bounds__(256)

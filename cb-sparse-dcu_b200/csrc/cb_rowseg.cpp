@@ -221,7 +221,8 @@ std::string build_rowseg(const DeviceLayout &L, int64_t warps, RowSegHost &R) {
     R.W = (int32_t)W;
     R.wbase.assign((size_t)G, 0);
     R.wlen.assign((size_t)G, 0);
-#pragma omp parallel
+    // (threads only where the sorts outweigh a parallel region's start)
+#pragma omp parallel if (nv >= (int64_t(1) << 22))
     {
         std::vector<int32_t> cols;
         std::vector<size_t> q;  // candidate first entries, their scores increasing

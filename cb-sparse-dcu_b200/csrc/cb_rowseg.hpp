@@ -19,10 +19,11 @@
 //
 // Chunks are grouped in SEGMENTS of M consecutive chunks, about one segment
 // per resident warp (equal entry counts: balanced by construction).  A row
-// that crosses segment boundaries is a SPAN: each of its segments leaves a
-// partial sum in a slot (2 s: the segment's first row, 2 s + 1: its last),
-// and the last segment to arrive on the span's counter adds the slots in
-// segment order and stores y, so results do not depend on timing.
+// that crosses segment boundaries is a SPAN.  Over one boundary its two parts
+// meet in an exchange word; over more, each segment leaves a partial sum in a
+// slot (2 s: the segment's first row, 2 s + 1: its last), and the last segment
+// to arrive on the span's counter adds the slots in segment order and stores
+// y; either way results do not depend on timing.
 // Each CTA also holds a WINDOW of x in shared memory: wlen[b] consecutive
 // columns from wbase[b], at most kRsWindowBytes, chosen on the host as the one
 // that saves the most gather traffic over its own staging (none where every

@@ -16,13 +16,17 @@
 //   * gathers x for its kRsK entries, all loads in flight at once: from the
 //     CTA's window of x in shared memory (staged at the start) when the
 //     entry's word says so, else from global memory,
-//   * counts its row starts; an exclusive warp scan of the counts gives the
-//     ordinal of the row it starts in,
+//   * counts the row starts of the lanes before it (one ballot per entry),
+//     which gives the ordinal of the row it starts in,
 //   * adds its entries along its rows in registers; a row that starts and
 //     ends inside the lane is stored at once,
 //   * joins the rows that run across lanes with one segmented inclusive scan
-//     (reset at lanes holding a row start), carrying the chunk's last row into
-//     the next chunk.
+//     (reset at lanes holding a row start, its steps' lanes read off the
+//     ballots, ended once no row reaches further), carrying the chunk's last
+//     row into the next chunk.
+// Bound by instruction issue and the gathers outside the window; with the row
+// starts and the scan's flags shuffled instead, n = 1048576, mean 16, FP64
+// took 56.8 us instead of 49.5, n = 300007, FP32 18.1 instead of 15.7.
 // The products of one row are added in entry order within a lane and in lane
 // order across lanes, fixed by the layout: results are bitwise reproducible
 // (the balanced schedule's atomics excepted).  The reference adds each entry

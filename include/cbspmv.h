@@ -70,10 +70,8 @@ typedef struct cbspmv_opts {
                              cb-spmv-dcu.hpp:1431-1433), 5 row segments (the
                              stored entries sorted by row in chunks of 128,
                              summed per lane and joined by one scan; built
-                             at upload, and the automatic choice, when every
-                             block is a COO block and values are stored;
-                             keeps a second copy of the values on the
-                             device), 6 balanced (plans built with row_owned
+                             at upload, and the automatic choice; keeps a
+                             second copy of the values on the device), 6 balanced (plans built with row_owned
                              = 0 and stored values: the entries in the
                              plan's block order, grouped as the reference's
                              CTAs, added into y with atomics as its
