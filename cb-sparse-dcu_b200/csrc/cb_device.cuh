@@ -203,6 +203,14 @@ __device__ __forceinline__ void add_csr_dense(const uint8_t *base, const uint4 b
     }
 }
 
+// First statement of a kernel launched with launch_behind (every thread): waits
+// until the launches before it on the stream have completed and their writes
+// are visible, then lets the next such launch be set up.
+__device__ __forceinline__ void behind_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ---- bulk asynchronous copies (TMA, no multicast) completing on mbarriers.
 // Every wait is bounded: after kWaitLimit polls it sets *err and gives up.
 constexpr uint32_t kWaitLimit = 1u << 22;

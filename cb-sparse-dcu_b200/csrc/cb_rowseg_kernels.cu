@@ -174,6 +174,7 @@ __device__ __forceinline__ void stage_wait() {
 template <typename T, bool UNIT, bool MAP>
 __global__ void __launch_bounds__(kRsWarps * 32, 1)
     cb_rowseg_kernel(const RowSegDev rs, const T *__restrict__ x, T *__restrict__ y) {
+    dev::behind_wait();
     using V = typename RsVec<T>::V;
     constexpr int K = kRsK, NV = RsVec<T>::n;
     constexpr int64_t CB = 32 * K * (4 + (UNIT ? 0 : (int64_t)sizeof(T)));
@@ -581,6 +582,7 @@ template <typename T, int G, bool UNIT>
 __global__ void __launch_bounds__(kRsWarps * 32, 1)
     cb_rowseg_mrhs_kernel(const RowSegDev rs, const T *__restrict__ x, T *__restrict__ y,
                           int nrhs, int64_t ldx, int64_t ldy, int xvec, int yvec) {
+    dev::behind_wait();
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     {  // rows without entries
         const int64_t total = (int64_t)rs.nempty * nrhs;
@@ -637,6 +639,7 @@ __global__ void __launch_bounds__(kRsBatchWarps * 32, 1)
                            const int4 *__restrict__ meta, int32_t nseg, uint32_t *sched,
                            const int2 *__restrict__ empty, int64_t nempty, const int4 *spans,
                            int32_t *counters, T *part, void *xch) {
+    dev::behind_wait();
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     for (int64_t i = ((int64_t)blockIdx.x * kRsBatchWarps + wib) * 32 + lane; i < nempty;
          i += (int64_t)gridDim.x * kRsBatchWarps * 32) {  // rows without entries
@@ -740,6 +743,27 @@ __global__ void cb_balanced_values_kernel(const BalancedDev b, const uint8_t *__
 
 }  // namespace
 
+// Launches a kernel that begins with dev::behind_wait: its blocks are set up
+// while the launch before it drains, so a call in a solver's loop does not pay
+// the launch latency between its kernels.  Calls one after another, without
+// and with: 256 x 256 grid, FP64 6.1 and 5.1 us; n = 300007, FP32 18.2 and
+// 16.0; uniform A x and A^T y 30.8 and 27.9.
+template <typename... P, typename... A>
+cudaError_t launch_behind(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem,
+                          cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 template <typename T, bool UNIT, bool MAP>
 const void *rowseg_fn() {
     return reinterpret_cast<const void *>(cb_rowseg_kernel<T, UNIT, MAP>);
@@ -758,9 +782,8 @@ cudaError_t launch_rowseg_m(const DevLayout &d, const void *x, void *y, size_t s
     while (keep < smem) keep *= 2;
     dev_resident_l1(fn, kRsWarps * 32, keep);
     // the grid the segments and windows were assigned for
-    cb_rowseg_kernel<T, UNIT, MAP><<<(unsigned)d.rs.G, kRsWarps * 32, smem, stream>>>(
-        d.rs, static_cast<const T *>(x), static_cast<T *>(y));
-    return cudaSuccess;
+    return launch_behind(cb_rowseg_kernel<T, UNIT, MAP>, (unsigned)d.rs.G, kRsWarps * 32, smem,
+                         stream, d.rs, static_cast<const T *>(x), static_cast<T *>(y));
 }
 
 template <typename T, bool UNIT>
@@ -801,8 +824,10 @@ cudaError_t launch_mrhs_g(const DevLayout &d, const T *x, T *y, int r, int64_t l
                           int xvec, int yvec, cudaStream_t stream) {
     const void *fn = reinterpret_cast<const void *>(cb_rowseg_mrhs_kernel<T, G, UNIT>);
     dev_resident_l1(fn, kRsWarps * 32, 0);  // sets the carveout: all L1
-    cb_rowseg_mrhs_kernel<T, G, UNIT><<<(unsigned)d.rs.G, kRsWarps * 32, 0, stream>>>(
-        d.rs, x, y, r, ldx, ldy, xvec, yvec);
+    const cudaError_t e =
+        launch_behind(cb_rowseg_mrhs_kernel<T, G, UNIT>, (unsigned)d.rs.G, kRsWarps * 32, 0,
+                      stream, d.rs, x, y, r, ldx, ldy, xvec, yvec);
+    if (e != cudaSuccess) return e;
     note_launch();
     return cudaGetLastError();
 }
@@ -947,14 +972,14 @@ cudaError_t launch_rowseg_batch(int f32, const RsBatchMat *mats, const int4 *seg
                                 cudaStream_t stream) {
     if (nwarps <= 0 || nwarps % kRsBatchWarps) return cudaErrorInvalidValue;
     const unsigned grid = (unsigned)(nwarps / kRsBatchWarps);
-    if (f32)
-        cb_rowseg_batch_kernel<float><<<grid, kRsBatchWarps * 32, 0, stream>>>(
-            mats, segs, meta, nseg, sched, empty, nempty, spans, counters,
-            static_cast<float *>(part), xch);
-    else
-        cb_rowseg_batch_kernel<double><<<grid, kRsBatchWarps * 32, 0, stream>>>(
-            mats, segs, meta, nseg, sched, empty, nempty, spans, counters,
-            static_cast<double *>(part), xch);
+    const cudaError_t e =
+        f32 ? launch_behind(cb_rowseg_batch_kernel<float>, grid, kRsBatchWarps * 32, 0, stream,
+                            mats, segs, meta, nseg, sched, empty, nempty, spans, counters,
+                            static_cast<float *>(part), xch)
+            : launch_behind(cb_rowseg_batch_kernel<double>, grid, kRsBatchWarps * 32, 0, stream,
+                            mats, segs, meta, nseg, sched, empty, nempty, spans, counters,
+                            static_cast<double *>(part), xch);
+    if (e != cudaSuccess) return e;
     note_launch();
     return cudaGetLastError();
 }
