@@ -51,25 +51,52 @@ template <typename T> struct RsVec;
 template <> struct RsVec<double> { using V = double2; static constexpr int n = 2; };
 template <> struct RsVec<float> { using V = float4; static constexpr int n = 4; };
 
+// Words and values of the stream.  The launch before may have written the
+// values (cbspmv_set_values), so the loads are coherent ones (see
+// launch_behind), and volatile, which keeps them after behind_wait's wait.
 __device__ __forceinline__ uint4 ld_stream(const uint4 *p, uint64_t pol) {
     uint4 r;
-    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0,%1,%2,%3}, [%4], %5;"
+    asm volatile("ld.global.L1::no_allocate.L2::cache_hint.v4.u32 {%0,%1,%2,%3}, [%4], %5;"
         : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
         : "l"(p), "l"(pol));
     return r;
 }
 __device__ __forceinline__ double2 ld_stream(const double2 *p, uint64_t pol) {
     double2 r;
-    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.f64 {%0,%1}, [%2], %3;"
+    asm volatile("ld.global.L1::no_allocate.L2::cache_hint.v2.f64 {%0,%1}, [%2], %3;"
         : "=d"(r.x), "=d"(r.y)
         : "l"(p), "l"(pol));
     return r;
 }
 __device__ __forceinline__ float4 ld_stream(const float4 *p, uint64_t pol) {
     float4 r;
-    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f32 {%0,%1,%2,%3}, [%4], %5;"
+    asm volatile("ld.global.L1::no_allocate.L2::cache_hint.v4.f32 {%0,%1,%2,%3}, [%4], %5;"
         : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w)
         : "l"(p), "l"(pol));
+    return r;
+}
+// Values of x, which the launch before may have written: the same loads, with
+// no hint.
+__device__ __forceinline__ double ld_x(const double *p) {
+    double r;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(r) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ float ld_x(const float *p) {
+    float r;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(r) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ double2 ld_x(const double2 *p) {
+    double2 r;
+    asm volatile("ld.global.v2.f64 {%0,%1}, [%2];" : "=d"(r.x), "=d"(r.y) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ float4 ld_x(const float4 *p) {
+    float4 r;
+    asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];"
+                 : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w)
+                 : "l"(p));
     return r;
 }
 __device__ __forceinline__ void unpack(const double2 &v, double *o) {
@@ -173,7 +200,7 @@ __device__ __forceinline__ void stage_wait() {
 
 template <typename T, bool UNIT, bool MAP>
 __global__ void __launch_bounds__(kRsWarps * 32, 1)
-    cb_rowseg_kernel(const RowSegDev rs, const T *__restrict__ x, T *__restrict__ y) {
+    cb_rowseg_kernel(const RowSegDev rs, const T *x, T *__restrict__ y) {
     dev::behind_wait();
     using V = typename RsVec<T>::V;
     constexpr int K = kRsK, NV = RsVec<T>::n;
@@ -248,7 +275,7 @@ __global__ void __launch_bounds__(kRsWarps * 32, 1)
 #pragma unroll
             for (int j = 0; j < K; ++j) {
                 const uint32_t col = w[j] & kRsColMask;
-                xv[j] = (w[j] & kRsWin) ? xs[(int)col - wb] : __ldg(x + col);
+                xv[j] = (w[j] & kRsWin) ? xs[(int)col - wb] : ld_x(x + col);
             }
             // row starts of the lanes before this one, and the lanes that hold
             // one, from one ballot per entry
@@ -377,13 +404,13 @@ __device__ __forceinline__ void rs_mrhs_segment(const RsMat<T> &A, int cb, int c
     auto load_x = [&](uint32_t col, T *o) {
         const T *px = A.x + (int64_t)col * A.ldx + c0;
         if (A.xvec) {
-            if (c0 < nrhs) unpack(__ldg(reinterpret_cast<const VT *>(px)), o);
+            if (c0 < nrhs) unpack(ld_x(reinterpret_cast<const VT *>(px)), o);
             else
 #pragma unroll
                 for (int k = 0; k < V; ++k) o[k] = T(0);
         } else {
 #pragma unroll
-            for (int k = 0; k < V; ++k) o[k] = c0 + k < nrhs ? __ldg(px + k) : T(0);
+            for (int k = 0; k < V; ++k) o[k] = c0 + k < nrhs ? ld_x(px + k) : T(0);
         }
     };
     auto store_y = [&](int64_t row, const T *v) {
@@ -580,7 +607,7 @@ __device__ __forceinline__ void rs_mrhs_segment(const RsMat<T> &A, int cb, int c
 
 template <typename T, int G, bool UNIT>
 __global__ void __launch_bounds__(kRsWarps * 32, 1)
-    cb_rowseg_mrhs_kernel(const RowSegDev rs, const T *__restrict__ x, T *__restrict__ y,
+    cb_rowseg_mrhs_kernel(const RowSegDev rs, const T *x, T *__restrict__ y,
                           int nrhs, int64_t ldx, int64_t ldy, int xvec, int yvec) {
     dev::behind_wait();
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -747,7 +774,11 @@ __global__ void cb_balanced_values_kernel(const BalancedDev b, const uint8_t *__
 // while the launch before it drains, so a call in a solver's loop does not pay
 // the launch latency between its kernels.  Calls one after another, without
 // and with: 256 x 256 grid, FP64 6.1 and 5.1 us; n = 300007, FP32 18.2 and
-// 16.0; uniform A x and A^T y 30.8 and 27.9.
+// 16.0; uniform A x and A^T y 30.8 and 27.9.  Such a kernel reads what a
+// launch before it may have written (x, the stream's values) by coherent
+// volatile loads (ld_x, ld_stream, stage_window): one through the read-only
+// path (__ldg) could be moved before behind_wait and need not see those
+// writes.  __ldg is for what stays as uploaded (words, meta, spans, row maps).
 template <typename... P, typename... A>
 cudaError_t launch_behind(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem,
                           cudaStream_t stream, A... args) {
