@@ -10,8 +10,8 @@
 #include <cstdlib>
 #include <cstring>
 #include <future>
-#include <new>
 #include <mutex>
+#include <new>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -1876,10 +1876,14 @@ cbspmv_status cbspmv_batch_graph_launch(cbspmv_batch *b, int per_matrix, void *s
         } else {  // fork into 8 branches, round-robin over the matrices, join
             cudaEventRecord(b->ev[8], b->cap[0]);
             for (int q = 1; q < 8; ++q) cudaStreamWaitEvent(b->cap[q], b->ev[8], 0);
+            // (the launches of a plan listed several times share its scratch:
+            // all on the branch of its first place)
             for (size_t k = 0; k < b->plans.size() && !crc; ++k) {
                 const cb::MatView &v = b->views[k];
+                const size_t q = (size_t)(std::find(b->plans.begin(), b->plans.end(),
+                                                    b->plans[k]) - b->plans.begin()) % 8;
                 crc = run_side(b->plans[k], b->plans[k]->A, v.x, v.y, v.nrhs, v.ldx, v.ldy,
-                               b->cap[k % 8]);
+                               b->cap[q]);
             }
             for (int q = 1; q < 8; ++q) {
                 cudaEventRecord(b->ev[q], b->cap[q]);

@@ -409,8 +409,8 @@ cbspmv_status cbspmv_batch_run_each(cbspmv_batch *batch, void *stream);
 
 /* Replays a CUDA graph held by the batch: per_matrix = 0 captures
  * cbspmv_batch_run, per_matrix = 1 captures the per-matrix launches spread
- * over 8 parallel branches.  Captured on first use (and after a re-bind),
- * then launched on `stream`. */
+ * over 8 parallel branches (those of one plan on one branch, in order).
+ * Captured on first use (and after a re-bind), then launched on `stream`. */
 cbspmv_status cbspmv_batch_graph_launch(cbspmv_batch *batch, int per_matrix,
                                         void *stream);
 

@@ -1,0 +1,61 @@
+"""Batches that list one plan several times (GPU): its launches share its
+scratch, so none of them may overlap another.  Rows over one segment boundary
+(exchange words) and over several (slots and a counter); the plan's own product
+afterwards is what it was before."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _coo(per_row, m=400, n=6000):
+    from cbspmv import gen
+    rng = np.random.default_rng(per_row)
+    cols = np.stack([np.sort(rng.choice(n, per_row, replace=False)) for _ in range(m)])
+    return gen.Coo(m, n, np.repeat(np.arange(m), per_row).astype(np.int32),
+                   cols.reshape(-1).astype(np.int32), rng.standard_normal(m * per_row))
+
+
+def _modes(batch):
+    return (("run", batch.run), ("run_each", batch.run_each),
+            ("graph", lambda: batch.graph_launch(False)),
+            ("graph_each", lambda: batch.graph_launch(True)))
+
+
+@pytest.mark.parametrize("per_row", [200, 900])
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("nrhs", [1, 5])
+def test_one_plan_on_every_entry(cuda, per_row, f32, nrhs):
+    import torch
+    import cbspmv
+    dt = torch.float32 if f32 else torch.float64
+    coo = _coo(per_row)
+    plan = cbspmv.Plan(coo, value_type=int(f32))
+    other = cbspmv.Plan(_coo(129), value_type=int(f32))
+    plans = [plan, plan, other, plan, other, plan, plan, plan, plan, plan, plan]
+    xs = [torch.randn(coo.n, nrhs, device=cuda, dtype=dt) for _ in plans]
+    ys = [torch.empty(coo.m, nrhs, device=cuda, dtype=dt) for _ in plans]
+
+    def own(p, x):  # a product of the plan by itself, waited for
+        y = p.spmv(x if nrhs > 1 else x[:, 0].contiguous()).reshape(-1, nrhs)
+        torch.cuda.synchronize()
+        return y
+
+    want = [own(p, x) for p, x in zip(plans, xs)]
+    scale = max(float(w.abs().max()) for w in want)
+    batch = cbspmv.Batch(plans, [nrhs] * len(plans)).bind(xs, ys)
+    for how, fn in _modes(batch):
+        for _ in range(3):
+            for y in ys:
+                y.fill_(float("nan"))
+            fn()
+            torch.cuda.synchronize()
+            for y, w in zip(ys, want):
+                # run_each and its graph launch the plan's own product; the one
+                # launch cuts other segments, so it adds in another order
+                if how.endswith("each"):
+                    assert torch.equal(y, w), how
+                else:
+                    tol = (1e-4 if f32 else 1e-12) * scale
+                    assert float((y - w).abs().max()) <= tol, how
+        assert torch.equal(own(plan, xs[0]), want[0]), how
