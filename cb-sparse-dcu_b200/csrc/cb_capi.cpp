@@ -1865,7 +1865,16 @@ cbspmv_status cbspmv_batch_graph_launch(cbspmv_batch *b, int per_matrix, void *s
         for (int q = 0; q < 9; ++q)
             if (!b->ev[q]) CB_CUDA(cudaEventCreateWithFlags(&b->ev[q], cudaEventDisableTiming),
                                    "create capture event");
-        // one eager run first: launchers configure their kernels on first use
+        // one eager run first: launchers configure their kernels on first use.
+        // It runs the plans, so it waits for what the caller has issued on them
+        // (a capturing stream has nothing in flight that it could wait for)
+        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &capturing) != cudaSuccess) {
+            cudaGetLastError();
+        } else if (capturing == cudaStreamCaptureStatusNone) {
+            CB_CUDA(cudaEventRecord(b->ev[8], static_cast<cudaStream_t>(stream)), "batch warm-up");
+            CB_CUDA(cudaStreamWaitEvent(b->cap[0], b->ev[8], 0), "batch warm-up");
+        }
         rc = mode ? batch_each(b, b->cap[0]) : batch_one(b, b->cap[0]);
         if (rc) return rc;
         CB_CUDA(cudaStreamSynchronize(b->cap[0]), "batch warm-up");

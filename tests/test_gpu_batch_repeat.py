@@ -59,3 +59,33 @@ def test_one_plan_on_every_entry(cuda, per_row, f32, nrhs):
                     tol = (1e-4 if f32 else 1e-12) * scale
                     assert float((y - w).abs().max()) <= tol, how
         assert torch.equal(own(plan, xs[0]), want[0]), how
+
+
+@pytest.mark.parametrize("per_matrix", [False, True])
+@pytest.mark.parametrize("ahead", ["own", "batch"])
+def test_first_graph_launch_waits_for_the_stream(cuda, per_matrix, ahead):
+    """The first graph launch runs the plans once before it captures them:
+    after the products already on the stream, not beside them."""
+    import torch
+    import cbspmv
+    coo = _coo(900, m=4000)
+    plan = cbspmv.Plan(coo)
+    x = torch.randn(coo.n, device=cuda, dtype=torch.float64)
+    want = plan.spmv(x)
+    torch.cuda.synchronize()
+    for _ in range(3):
+        y = torch.empty_like(want)
+        xs, ys = [x[:, None].contiguous()], [torch.empty(coo.m, 1, device=cuda, dtype=x.dtype)]
+        batch = cbspmv.Batch([plan], [1]).bind(xs, ys)
+        batch.run()
+        torch.cuda.synchronize()
+        once = ys[0].clone()
+        for _ in range(300):
+            plan.spmv(x, y) if ahead == "own" else batch.run()
+        batch.graph_launch(per_matrix)
+        torch.cuda.synchronize()
+        assert torch.equal(ys[0][:, 0], want) if per_matrix else torch.equal(ys[0], once)
+        assert ahead == "batch" or torch.equal(y, want)
+        assert torch.equal(plan.spmv(x), want)
+        batch.run()
+        assert torch.equal(ys[0], once)
