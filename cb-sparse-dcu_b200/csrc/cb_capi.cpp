@@ -65,6 +65,11 @@ struct DevSide {
     uint32_t *dunit = nullptr;
     int64_t *ustart = nullptr;
     int partial_nrhs = 0;
+    // partials that were too small for a later call: graphs captured before it
+    // and bound batches still use them.  Each is at least twice the one before,
+    // so together they are smaller than the one in use.
+    void *old_partials[32] = {};
+    int nold = 0;
     int64_t *vsrc_ptr = nullptr;
     int32_t *vsrc = nullptr;
     bool one_source = false;        // every stored value has one input: vsrc and
@@ -90,6 +95,7 @@ struct DevSide {
                       pat[0], pat[1], pat[2], pat[3]};
         for (void *p : ps)
             if (p) cudaFree(p);
+        while (nold > 0) cudaFree(old_partials[--nold]);
         for (void *&q : rs) {
             if (q) cudaFree(q);
             q = nullptr;
@@ -463,14 +469,18 @@ cbspmv_status upload_patterns(DevSide &s, const cb::HostCB &g, cudaStream_t st) 
     return CBSPMV_OK;
 }
 
-// Partial slots sized for nrhs right-hand sides.
+// Partial slots for nrhs right-hand sides at least; smaller ones are kept until
+// the plan is destroyed (see DevSide::old_partials).
 cbspmv_status ensure_partials(DevSide &s, int nrhs, size_t vsz) {
     if (s.lay.slots == 0 || s.partial_nrhs >= nrhs) return CBSPMV_OK;
-    if (s.partials) cudaFree(s.partials);
-    s.partials = nullptr;
-    const size_t bytes = (size_t)s.lay.slots * nrhs * s.lay.bs * vsz;
-    CB_CUDA(cudaMalloc(&s.partials, bytes), "allocate split-row partials");
-    s.partial_nrhs = nrhs;
+    const int64_t want = std::min<int64_t>(std::max<int64_t>(nrhs, 2 * (int64_t)s.partial_nrhs),
+                                           INT32_MAX);
+    void *fresh = nullptr;
+    CB_CUDA(cudaMalloc(&fresh, (size_t)s.lay.slots * (size_t)want * s.lay.bs * vsz),
+            "allocate split-row partials");
+    if (s.partials) s.old_partials[s.nold++] = s.partials;
+    s.partials = fresh;
+    s.partial_nrhs = (int)want;
     s.d.partials = s.partials;
     return CBSPMV_OK;
 }
