@@ -1517,6 +1517,11 @@ struct cbspmv_batch {
     uint32_t *d_sched = nullptr;    // 2 scheduler words (unit counter, warps out)
     uint32_t *herr = nullptr, *derr = nullptr;  // error word (host-mapped)
     uint32_t tile_cap = 16;         // shared buffer bytes: every plan's largest tile
+    // over the tiles: arrival counters and split-row partials of every entry,
+    // its own (one plan may be listed several times), at these byte offsets
+    void *d_scratch = nullptr;
+    size_t counter_bytes = 0;       // of all entries, at the start
+    std::vector<size_t> coff, poff;
     cudaStream_t cap[8] = {};
     cudaEvent_t ev[9] = {};
     cudaGraphExec_t exec[2] = {};
@@ -1543,7 +1548,7 @@ struct cbspmv_batch {
         for (void *p : {(void *)d_toff, (void *)d_ustart, (void *)d_uorder, (void *)d_sched,
                         (void *)d_views, (void *)d_rmats, (void *)d_rsegs, (void *)d_rmeta,
                         (void *)d_rspans, (void *)d_rsched, (void *)d_rcnt, (void *)d_rempty,
-                        d_rpart, d_rxch})
+                        d_rpart, d_rxch, d_scratch})
             if (p) cudaFree(p);
         if (herr) cudaFreeHost(herr);
     }
@@ -1552,16 +1557,15 @@ struct cbspmv_batch {
 namespace {
 
 // Reports (once) that a batch launch gave up a bounded device wait, and
-// resets the plans' arrival counters and the batch's scheduler words.
+// resets the batch's arrival counters and scheduler words.
 cbspmv_status batch_device_error(cbspmv_batch *b, cudaStream_t st) {
     if (!b->herr) return CBSPMV_OK;
     volatile uint32_t *w = b->herr;
     if (*w == 0) return CBSPMV_OK;
     *w = 0;
-    for (cbspmv_plan *p : b->plans)
-        if (p->A.counters)
-            CB_CUDA(cudaMemsetAsync(p->A.counters, 0, (p->A.lay.gb_m + 4) * sizeof(int32_t), st),
-                    "reset scratch after a device error");
+    if (b->d_scratch)
+        CB_CUDA(cudaMemsetAsync(b->d_scratch, 0, b->counter_bytes, st),
+                "reset scratch after a device error");
     CB_CUDA(cudaMemsetAsync(b->d_sched, 0, 16, st), "reset scratch after a device error");
     return fail(CBSPMV_ERR_DEVICE,
                 "a bounded device wait gave up in an earlier batch launch: its outputs are "
@@ -1667,6 +1671,38 @@ cbspmv_status batch_rowseg_setup(cbspmv_batch *b, const int *nrhs) {
     b->nrempty = (int64_t)empty.size();
     b->rs_mode = true;
     return CBSPMV_OK;
+}
+
+// Entry k's view over the tiles, on the batch's own scratch.
+cb::MatView batch_view(const cbspmv_batch *b, size_t k, const void *x, void *y, int nrhs) {
+    cb::MatView v = cb::mat_view(b->plans[k]->A.d, x, y, nrhs, nrhs, nrhs);
+    if (b->d_scratch) {
+        char *base = static_cast<char *>(b->d_scratch);
+        v.counters = reinterpret_cast<int32_t *>(base + b->coff[k]);
+        v.partials = base + b->poff[k];
+    }
+    return v;
+}
+
+// That scratch, when the batch runs over the tiles.
+cbspmv_status batch_scratch(cbspmv_batch *b) {
+    if (b->rs_mode) return CBSPMV_OK;
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        const size_t a = at;
+        at += (bytes + 255) & ~size_t(255);
+        return a;
+    };
+    for (cbspmv_plan *p : b->plans) b->coff.push_back(take(p->A.lay.gb_m * sizeof(int32_t)));
+    b->counter_bytes = at;
+    for (size_t k = 0; k < b->plans.size(); ++k) {
+        const cb::DeviceLayout &L = b->plans[k]->A.lay;
+        b->poff.push_back(take((size_t)L.slots * b->views[k].nrhs * L.bs * (b->f32 ? 4 : 8)));
+    }
+    cudaError_t e = cudaMalloc(&b->d_scratch, std::max<size_t>(at, 16));
+    if (e == cudaSuccess) e = cudaMemset(b->d_scratch, 0, std::max<size_t>(b->counter_bytes, 16));
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+    return e == cudaSuccess ? CBSPMV_OK : cuda_fail(e, "allocate batch scratch");
 }
 
 // One persistent launch over every matrix of the batch.
@@ -1804,7 +1840,9 @@ cbspmv_status cbspmv_batch_create(cbspmv_plan *const *plans, int count, const in
         delete b;
         return cuda_fail(e, "allocate batch tables");
     }
-    if (cbspmv_status rc = batch_rowseg_setup(b, nrhs)) {
+    cbspmv_status rc = batch_rowseg_setup(b, nrhs);
+    if (!rc) rc = batch_scratch(b);
+    if (rc) {
         delete b;
         return rc;
     }
@@ -1822,7 +1860,7 @@ cbspmv_status cbspmv_batch_bind(cbspmv_batch *b, const void *const *x, void *con
         if ((s.lay.m > 0 && !y[k]) || (s.lay.n > 0 && !x[k]))
             return fail(CBSPMV_ERR_INVALID, "null x or y in batch");
         cb::MatView &v = b->views[k];
-        v = cb::mat_view(s.d, x[k], y[k], v.nrhs, v.nrhs, v.nrhs);
+        v = batch_view(b, k, x[k], y[k], v.nrhs);
     }
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     CB_CUDA(cudaMemcpyAsync(b->d_views, b->views.data(), b->views.size() * sizeof(cb::MatView),

@@ -386,8 +386,8 @@ cbspmv_status cbspmv_tune(const cbspmv_coo *coo, const cbspmv_opts *opts, int nr
  * batch launch runs every matrix, whatever its size and right-hand-side
  * count, in ONE persistent kernel: its warps take scheduling units of the
  * matrices' concatenated tiles from a device counter (the units are cut here
- * for the current device).  A plan may belong to several batches but is run
- * by one of them (or by itself) at a time. */
+ * for the current device).  A plan may be listed several times and belong to
+ * several batches, but is run by one of them (or by itself) at a time. */
 typedef struct cbspmv_batch cbspmv_batch;
 
 cbspmv_status cbspmv_batch_create(cbspmv_plan *const *plans, int count,

@@ -61,6 +61,37 @@ def test_one_plan_on_every_entry(cuda, per_row, f32, nrhs):
         assert torch.equal(own(plan, xs[0]), want[0]), how
 
 
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("nrhs", [1, 5, 20])
+def test_one_plan_on_every_entry_over_tiles(cuda, f32, nrhs):
+    """The same over the tiles, with block rows split over several (their
+    partial sums and arrival counters are the entry's own), and after a
+    product with more right-hand sides has given the plan larger partials."""
+    import torch
+    import cbspmv
+    import cbdump as cd
+    dt = torch.float32 if f32 else torch.float64
+    coo = _coo(200)
+    plan = cbspmv.Plan(coo, value_type=int(f32), kernel=3, tile_entries=64)
+    assert plan.info()["split_rows"] > 0
+    plans = [plan] * 6
+    X = [torch.randn(coo.n, nrhs, device=cuda, dtype=dt) for _ in plans]
+    ys = [torch.empty(coo.m, nrhs, device=cuda, dtype=dt) for _ in plans]
+    refs = [cd.oracle_spmm_ld(coo, np.ascontiguousarray(x.cpu().numpy().astype(np.float64).T))
+            for x in X]
+    batch = cbspmv.Batch(plans, [nrhs] * len(plans)).bind(X, ys)
+    for rep in range(2):
+        for how, fn in _modes(batch):
+            for y in ys:
+                y.fill_(float("nan"))
+            fn()
+            torch.cuda.synchronize()
+            for y, (ref, ab) in zip(ys, refs):
+                tol = 1e-5 if f32 else 1e-12
+                assert np.all(np.abs(y.cpu().numpy().T - ref) <= tol * ab + 1e-30), (how, rep)
+        plan.spmv(torch.randn(coo.n, 3 * nrhs, device=cuda, dtype=dt))
+
+
 @pytest.mark.parametrize("per_matrix", [False, True])
 @pytest.mark.parametrize("ahead", ["own", "batch"])
 def test_first_graph_launch_waits_for_the_stream(cuda, per_matrix, ahead):
