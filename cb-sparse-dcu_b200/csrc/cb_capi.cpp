@@ -869,8 +869,9 @@ cbspmv_status cbspmv_autotune_ex(cbspmv_plan *p, int nrhs, void *stream, int *ke
         return cuda_fail(e, "autotune scratch");
     }
     const int keep = s.d.kernel, keep_rl = s.d.rl;
+    const int own = cb::auto_kernel(s.d, nrhs);  // the automatic choice
     int best = -1, best_rl = 0;
-    float best_ms = 0.f;
+    float best_ms = 0.f, own_ms = -1.f;
     for (const auto &c : cands) {
         s.d.kernel = c.first;
         s.d.rl = c.second;
@@ -890,6 +891,7 @@ cbspmv_status cbspmv_autotune_ex(cbspmv_plan *p, int nrhs, void *stream, int *ke
         float t = 0.f;
         cudaEventElapsedTime(&t, e0, e1);
         t /= reps;
+        if (c.first == own && c.second == 0) own_ms = t;
         if (best < 0 || t < best_ms) {
             best = c.first;
             best_rl = c.second;
@@ -897,6 +899,14 @@ cbspmv_status cbspmv_autotune_ex(cbspmv_plan *p, int nrhs, void *stream, int *ke
         }
     }
     cleanup();
+    // the automatic choice wins a tie: ten launches are told apart to about
+    // 0.3 us and 1%, and where launching bounds several kernels alike (4.4 us
+    // for 100,000 unit values) the fastest of them is chance
+    if (own_ms >= 0 && best_ms > 0.99f * own_ms - 0.0003f) {
+        best = own;
+        best_rl = 0;
+        best_ms = own_ms;
+    }
     s.d.kernel = best;
     s.d.rl = best_rl;
     p->opts.kernel = best;

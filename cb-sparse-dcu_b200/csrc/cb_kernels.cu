@@ -852,31 +852,41 @@ bool use_pattern(const DevLayout &d) {
     return d.kernel == 4 || (d.kernel == 0 && d.pat_auto);
 }
 
+// The kernel (the numbers of the plan's kernel option) that runs y = A x.
+// Pattern reuse and the balanced schedule (plans built with row_owned = 0, the
+// reference's non-row-owned mode) take one right-hand side of unit stride.
+// The row-segment stream: when chosen, and the automatic choice except in
+// the reference's small-direct case.  It stores up to 4 bytes an entry
+// more than CSR and DENSE blocks do, but has no work per block: on
+// stencils (FP64, 3 unknowns a node) 24 us against the direct kernel's 46
+// at n = 98304 and 5.7 against 17 at n = 3000, on bands of 129 19 against
+// 43, on a dense 2000 x 2000 matrix 16 against 69 (the streaming kernel:
+// 35, 16, 20 and 30); FP32 and 32 x 32 blocks likewise
+int kernel_for(const DevLayout &d, int nrhs, int64_t ldx, int64_t ldy) {
+    const bool one = nrhs == 1 && ldx == 1 && ldy == 1;
+    if (one && use_pattern(d)) return 4;
+    if (one && d.bal.rows && (d.kernel == 6 || d.kernel == 0)) return 6;
+    if (d.rs.chunks &&
+        (d.kernel == 5 || (d.kernel == 0 && !d.small_direct && !use_pattern(d))))
+        return 5;
+    if (one && use_stream(d)) return 1;
+    return nrhs > 1 || d.kernel == 3 || d.kernel == 4 ? 3 : 2;
+}
+
 template <typename T, int BS>
 cudaError_t launch_tiles(const DevLayout &d, const void *x, void *y, int nrhs,
                          int64_t ldx, int64_t ldy, cudaStream_t stream) {
-    if (nrhs == 1 && ldx == 1 && ldy == 1 && use_pattern(d))
-        return launch_pattern_v<T>(d, x, y, stream);
-    // the row-segment stream: when chosen, and the automatic choice except in
-    // the reference's small-direct case.  It stores up to 4 bytes an entry
-    // more than CSR and DENSE blocks do, but has no work per block: on
-    // stencils (FP64, 3 unknowns a node) 24 us against the direct kernel's 46
-    // at n = 98304 and 5.7 against 17 at n = 3000, on bands of 129 19 against
-    // 43, on a dense 2000 x 2000 matrix 16 against 69 (the streaming kernel:
-    // 35, 16, 20 and 30); FP32 and 32 x 32 blocks likewise
-    const bool one = nrhs == 1 && ldx == 1 && ldy == 1;
-    // the balanced schedule: plans built with row_owned = 0 (the reference's
-    // non-row-owned mode), one right-hand side
-    if (one && d.bal.rows && (d.kernel == 6 || d.kernel == 0))
-        return launch_balanced(d, x, y, stream);
-    if (d.rs.chunks && (d.kernel == 5 || (d.kernel == 0 && !d.small_direct &&
-                                          !use_pattern(d))))
-        return one ? launch_rowseg(d, x, y, stream)
-                   : launch_rowseg_mrhs(d, x, y, nrhs, ldx, ldy, stream);
-    if (nrhs == 1 && ldx == 1 && ldy == 1 && use_stream(d))
-        return launch_stream<T, BS>(d, x, y, stream);
-    if (nrhs > 1 || d.kernel == 3 || d.kernel == 4)
-        return launch_spmm(d, x, y, nrhs, ldx, ldy, stream);
+    switch (kernel_for(d, nrhs, ldx, ldy)) {
+        case 4: return launch_pattern_v<T>(d, x, y, stream);
+        case 6: return launch_balanced(d, x, y, stream);
+        case 5:
+            return nrhs == 1 && ldx == 1 && ldy == 1
+                       ? launch_rowseg(d, x, y, stream)
+                       : launch_rowseg_mrhs(d, x, y, nrhs, ldx, ldy, stream);
+        case 1: return launch_stream<T, BS>(d, x, y, stream);
+        case 3: return launch_spmm(d, x, y, nrhs, ldx, ldy, stream);
+        default: break;
+    }
     switch (chunk_choice()) {
         case 4: return launch_chunk<T, BS, 4>(d, x, y, nrhs, ldx, ldy, stream);
         case 6: return launch_chunk<T, BS, 6>(d, x, y, nrhs, ldx, ldy, stream);
@@ -897,6 +907,12 @@ std::vector<uint32_t> direct_units(const uint32_t *tile8, int64_t ntiles) {
     }
     us.push_back((uint32_t)ntiles);
     return us;
+}
+
+int auto_kernel(const DevLayout &d, int nrhs) {
+    DevLayout f = d;
+    f.kernel = 0;
+    return kernel_for(f, nrhs, nrhs, nrhs);
 }
 
 int64_t kernel_launches() { return g_kernel_launches.load(); }

@@ -223,6 +223,9 @@ cudaError_t launch_rowseg_batch(int f32, const RsBatchMat *mats, const int4 *seg
                                 int32_t *counters, void *part, void *xch,
                                 cudaStream_t stream);
 
+// The automatic choice (kernel option 0) for nrhs contiguous right-hand sides.
+int auto_kernel(const DevLayout &d, int nrhs);
+
 // y = A x; x: n rows, y: m rows, row-major with leading dims for nrhs > 1.
 cudaError_t launch_spmv(const DevLayout &d, const void *x, void *y, int nrhs,
                         int64_t ldx, int64_t ldy, cudaStream_t stream);
