@@ -82,6 +82,7 @@ struct DevSide {
     // exchange words
     void *rs[11] = {};
     int64_t rs_bytes = 0;
+    size_t rs_nspan = 0;
     std::vector<int32_t> rs_cinfo;  // per chunk summaries (batches cut their own segments)
     std::vector<int32_t> rs_empty;  // rows without entries
     std::vector<int32_t> rs_vpos;   // per stored value: its stream entry (-1: none)
@@ -127,11 +128,17 @@ struct DevSide {
 
 // Pipelined host-buffer calls (cbspmv_spmv_host_async): copy in, compute and
 // copy out on three streams of their own, two sets of device buffers, so call
-// i+1's copy in overlaps call i's kernel and call i-1's copy out.
+// i+1's copy in overlaps call i's kernel and call i-1's copy out.  The kernels
+// run beside whatever the caller issued on its stream, products of the same
+// plan among it, so they have scratch of their own: scheduler words and
+// arrival counters, split-row partials, and the stream's span counters, slots
+// and exchange words, at these byte offsets.
 struct HostPipe {
     cudaStream_t in = nullptr, comp = nullptr, out = nullptr;
+    char *scratch = nullptr;
+    size_t partials = 0, span_counters = 0, part = 0, xch = 0;
+    int nrhs = 0;               // that the scratch and the buffers hold
     void *x[2] = {}, *y[2] = {};
-    size_t xb = 0, yb = 0;  // bytes of each buffer
     // x_ready: copy in done; x_free: kernel done reading x; y_ready: kernel
     // done writing y; y_free: copy out done
     cudaEvent_t x_ready[2] = {}, x_free[2] = {}, y_ready[2] = {}, y_free[2] = {};
@@ -146,9 +153,11 @@ struct HostPipe {
                 if (*e) cudaEventDestroy(*e), *e = nullptr;
             used[b] = false;
         }
+        if (scratch) cudaFree(scratch);
+        scratch = nullptr;
+        nrhs = 0;
         for (cudaStream_t *st : {&in, &comp, &out})
             if (*st) cudaStreamDestroy(*st), *st = nullptr;
-        xb = yb = 0;
     }
 };
 
@@ -415,6 +424,7 @@ cbspmv_status upload_rowseg(DevSide &s, int kernel, cudaStream_t st) {
     d.unit = R.unit;
     s.rs_bytes = (int64_t)(R.chunks.size() + 4 * (R.meta.size() + R.spans.size() +
                                                   R.rowmap.size() + R.empty.size()));
+    s.rs_nspan = R.spans.size() / 4;
     s.rs_cinfo = std::move(R.cinfo);
     s.rs_empty = std::move(R.empty);
     s.rs_vpos = std::move(R.vpos);
@@ -499,6 +509,11 @@ cbspmv_status take_device_error(cbspmv_plan *p, int side, cudaStream_t st) {
             cudaMemsetAsync(s.counters, 0, (s.lay.gb_m + 4) * sizeof(int32_t), st);
         if (e != cudaSuccess) return cuda_fail(e, "reset scratch after a device error");
     }
+    if (side == 0 && p->pipe.scratch) {
+        const cudaError_t e = cudaMemsetAsync(
+            p->pipe.scratch, 0, (s.lay.gb_m + 4) * sizeof(int32_t), p->pipe.comp);
+        if (e != cudaSuccess) return cuda_fail(e, "reset scratch after a device error");
+    }
     return fail(CBSPMV_ERR_DEVICE,
                 std::string("a bounded device wait gave up in an earlier launch on this plan (") +
                     (side ? "A^T" : "A") +
@@ -511,8 +526,10 @@ cbspmv_status device_errors(cbspmv_plan *p, cudaStream_t st) {
     return rc ? rc : rt;
 }
 
+// (own: on the host pipe's scratch, else on the plan's)
 cbspmv_status run_side(cbspmv_plan *p, DevSide &s, const void *x, void *y,
-                       int nrhs, int64_t ldx, int64_t ldy, cudaStream_t st) {
+                       int nrhs, int64_t ldx, int64_t ldy, cudaStream_t st,
+                       const HostPipe *own = nullptr) {
     if (!p->uploaded) return fail(CBSPMV_ERR_STATE, "plan not uploaded");
     if (cbspmv_status rc = take_device_error(p, &s == &p->AT ? 1 : 0, st)) return rc;
     if (nrhs < 1) return fail(CBSPMV_ERR_INVALID, "nrhs must be >= 1");
@@ -522,13 +539,55 @@ cbspmv_status run_side(cbspmv_plan *p, DevSide &s, const void *x, void *y,
         return fail(CBSPMV_ERR_INVALID, "leading dimension smaller than nrhs");
     if ((s.lay.m > 0 && !y) || (s.lay.n > 0 && !x && s.lay.nvals > 0))
         return fail(CBSPMV_ERR_INVALID, "null x or y");
-    cbspmv_status rc = ensure_partials(s, nrhs, vsize(p));
-    if (rc) return rc;
+    if (!own)
+        if (cbspmv_status rc = ensure_partials(s, nrhs, vsize(p))) return rc;
     int dev = -1;
     cudaGetDevice(&dev);
     if (dev != p->device)
         return fail(CBSPMV_ERR_STATE, "plan was uploaded to another device");
-    CB_CUDA(cb::launch_spmv(s.d, x, y, nrhs, ldx, ldy, st), "spmv launch");
+    if (!own) {
+        CB_CUDA(cb::launch_spmv(s.d, x, y, nrhs, ldx, ldy, st), "spmv launch");
+        return CBSPMV_OK;
+    }
+    cb::DevLayout d = s.d;
+    d.sched = reinterpret_cast<uint32_t *>(own->scratch);
+    d.counters = reinterpret_cast<int32_t *>(own->scratch) + 4;
+    d.partials = own->scratch + own->partials;
+    d.rs.counters = reinterpret_cast<int32_t *>(own->scratch + own->span_counters);
+    d.rs.part = own->scratch + own->part;
+    d.rs.xch = own->scratch + own->xch;
+    CB_CUDA(cb::launch_spmv(d, x, y, nrhs, ldx, ldy, st), "spmv launch");
+    return CBSPMV_OK;
+}
+
+// The host pipe's scratch for side s and nrhs right-hand sides.
+cbspmv_status pipe_scratch(HostPipe &q, const DevSide &s, int nrhs) {
+    const size_t vsz = s.lay.f32 ? 4 : 8;
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        const size_t a = at;
+        at += (std::max<size_t>(bytes, 16) + 255) & ~size_t(255);
+        return a;
+    };
+    take((s.lay.gb_m + 4) * sizeof(int32_t));
+    q.span_counters = take(s.rs_nspan * sizeof(int32_t));
+    const size_t zeroed = at;
+    q.partials = take((size_t)s.lay.slots * nrhs * s.lay.bs * vsz);
+    q.part = take(2 * (size_t)s.d.rs.nseg * cb::kRsSlotValues * vsz);
+    std::vector<uint32_t> words;
+    try {
+        words = empty_words(s.rs_nspan, vsz);
+    } catch (const std::bad_alloc &) {
+        return fail(CBSPMV_ERR_ALLOC, "out of host memory");
+    }
+    q.xch = take(words.size() * 4);
+    CB_CUDA(cudaMalloc((void **)&q.scratch, at), "allocate host pipeline scratch");
+    CB_CUDA(cudaMemsetAsync(q.scratch, 0, zeroed, q.comp), "clear host pipeline scratch");
+    CB_CUDA(cudaMemcpyAsync(q.scratch + q.xch, words.data(), words.size() * 4,
+                            cudaMemcpyHostToDevice, q.comp),
+            "clear host pipeline scratch");
+    CB_CUDA(cudaStreamSynchronize(q.comp), "clear host pipeline scratch");
+    q.nrhs = nrhs;
     return CBSPMV_OK;
 }
 
@@ -1020,7 +1079,7 @@ cbspmv_status cbspmv_spmv_host_async(cbspmv_plan *p, const void *x_host, void *y
     const cudaStream_t user = static_cast<cudaStream_t>(stream);
     const size_t xb = (size_t)p->host.n * nrhs * vsize(p);
     const size_t yb = (size_t)p->host.m * nrhs * vsize(p);
-    if (!q.comp || xb > q.xb || yb > q.yb) {  // set up, or grow for more rhs
+    if (!q.scratch || nrhs > q.nrhs) {  // set up, or grow for more rhs
         if (q.comp) {
             CB_CUDA(cudaStreamSynchronize(q.out), "drain host pipeline");
             CB_CUDA(cudaStreamSynchronize(q.comp), "drain host pipeline");
@@ -1034,8 +1093,7 @@ cbspmv_status cbspmv_spmv_host_async(cbspmv_plan *p, const void *x_host, void *y
             for (cudaEvent_t *e : {&q.x_ready[b], &q.x_free[b], &q.y_ready[b], &q.y_free[b]})
                 CB_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "create event");
         }
-        q.xb = std::max<size_t>(16, xb);
-        q.yb = std::max<size_t>(16, yb);
+        if ((rc = pipe_scratch(q, p->A, nrhs))) return rc;
     }
     const int b = (int)(q.calls & 1);
     // copy in (x_host holds the input now), after the kernel that last read
@@ -1047,7 +1105,7 @@ cbspmv_status cbspmv_spmv_host_async(cbspmv_plan *p, const void *x_host, void *y
     // compute, once x is in and the previous copy out of this y is done
     CB_CUDA(cudaStreamWaitEvent(q.comp, q.x_ready[b], 0), "wait");
     if (q.used[b]) CB_CUDA(cudaStreamWaitEvent(q.comp, q.y_free[b], 0), "wait");
-    rc = run_side(p, p->A, q.x[b], q.y[b], nrhs, nrhs, nrhs, q.comp);
+    rc = run_side(p, p->A, q.x[b], q.y[b], nrhs, nrhs, nrhs, q.comp, &q);
     if (rc) return rc;
     CB_CUDA(cudaEventRecord(q.x_free[b], q.comp), "record");
     CB_CUDA(cudaEventRecord(q.y_ready[b], q.comp), "record");
