@@ -138,6 +138,7 @@ struct HostPipe {
     char *scratch = nullptr;
     size_t partials = 0, span_counters = 0, part = 0, xch = 0;
     int nrhs = 0;               // that the scratch and the buffers hold
+    cudaEvent_t values = nullptr;  // a value update on the caller's stream
     void *x[2] = {}, *y[2] = {};
     // x_ready: copy in done; x_free: kernel done reading x; y_ready: kernel
     // done writing y; y_free: copy out done
@@ -156,6 +157,7 @@ struct HostPipe {
         if (scratch) cudaFree(scratch);
         scratch = nullptr;
         nrhs = 0;
+        if (values) cudaEventDestroy(values), values = nullptr;
         for (cudaStream_t *st : {&in, &comp, &out})
             if (*st) cudaStreamDestroy(*st), *st = nullptr;
     }
@@ -172,6 +174,7 @@ struct cbspmv_plan {
     void *hx = nullptr, *hy = nullptr;
     size_t hx_bytes = 0, hy_bytes = 0;
     HostPipe pipe;
+    bool values_new = true;  // set_values since the pipe last waited for it
     // loaded from an SpMV-only plan file: no per-value arrays, no host block
     // arrays; counts = the block counts the plan's info reports
     bool spmv_only = false;
@@ -1093,6 +1096,7 @@ cbspmv_status cbspmv_spmv_host_async(cbspmv_plan *p, const void *x_host, void *y
             for (cudaEvent_t *e : {&q.x_ready[b], &q.x_free[b], &q.y_ready[b], &q.y_free[b]})
                 CB_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "create event");
         }
+        CB_CUDA(cudaEventCreateWithFlags(&q.values, cudaEventDisableTiming), "create event");
         if ((rc = pipe_scratch(q, p->A, nrhs))) return rc;
     }
     const int b = (int)(q.calls & 1);
@@ -1102,7 +1106,13 @@ cbspmv_status cbspmv_spmv_host_async(cbspmv_plan *p, const void *x_host, void *y
     if (q.used[b]) CB_CUDA(cudaStreamWaitEvent(q.in, q.x_free[b], 0), "wait");
     if (xb) CB_CUDA(cudaMemcpyAsync(q.x[b], x_host, xb, cudaMemcpyHostToDevice, q.in), "copy x");
     CB_CUDA(cudaEventRecord(q.x_ready[b], q.in), "record");
-    // compute, once x is in and the previous copy out of this y is done
+    // compute, once x is in, the previous copy out of this y is done and the
+    // caller's last value update is
+    if (p->values_new) {
+        CB_CUDA(cudaEventRecord(q.values, user), "record");
+        CB_CUDA(cudaStreamWaitEvent(q.comp, q.values, 0), "wait");
+        p->values_new = false;
+    }
     CB_CUDA(cudaStreamWaitEvent(q.comp, q.x_ready[b], 0), "wait");
     if (q.used[b]) CB_CUDA(cudaStreamWaitEvent(q.comp, q.y_free[b], 0), "wait");
     rc = run_side(p, p->A, q.x[b], q.y[b], nrhs, nrhs, nrhs, q.comp, &q);
@@ -1353,6 +1363,7 @@ cbspmv_status cbspmv_set_values(cbspmv_plan *p, const void *input_values,
                     "this plan stores no values (every value was 1); build it with "
                     "keep_values = 1 to change them");
     cudaStream_t st = (cudaStream_t)stream;
+    p->values_new = true;
     auto side = [](const DevSide &s) {
         cb::ValueSide v;
         v.nvals = s.lay.nvals;

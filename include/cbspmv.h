@@ -218,9 +218,10 @@ cbspmv_status cbspmv_spmv_host(cbspmv_plan *plan, const void *x_host,
  * waits for this call's copy out; synchronize it before reading y_host, and
  * keep x_host unchanged and both buffers alive until then (pinned host memory
  * lets the copies run asynchronously).  The kernel may run beside other
- * products of the plan issued to `stream` before (it has scratch of its own).
- * The first call, and a call with more right-hand sides than before, allocates
- * the device buffers and that scratch.  No counterpart in the reference (its cb_spmv copies, runs
+ * products of the plan issued to `stream` before (it has scratch of its own),
+ * but after the cbspmv_set_values calls made before.  The first call, and a
+ * call with more right-hand sides than before, allocates the device buffers
+ * and that scratch.  No counterpart in the reference (its cb_spmv copies, runs
  * and copies back one call at a time). */
 cbspmv_status cbspmv_spmv_host_async(cbspmv_plan *plan, const void *x_host,
                                      void *y_host, int nrhs, void *stream);

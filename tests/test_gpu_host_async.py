@@ -1,5 +1,6 @@
 """cbspmv_spmv_host_async beside other work on the caller's stream (GPU): its
-kernels run on a stream of the plan's own, with scratch of their own.  Rows over one segment boundary (exchange words), over
+kernels run on a stream of the plan's own, with scratch of their own, after the
+caller's value updates.  Rows over one segment boundary (exchange words), over
 several (slots and counters), and split block rows over the tiles."""
 import ctypes
 
@@ -56,3 +57,28 @@ def test_beside_products_of_the_plan(cuda, per_row, kernel, f32, nrhs):
         assert all(torch.equal(yh, want.cpu()) for yh in yhs)
     plan.spmv(x, y)
     assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("f32", [False, True])
+def test_after_new_values(cuda, f32):
+    import torch
+    coo, plan = _plan(900, f32, 0)
+    dt = torch.float32 if f32 else torch.float64
+    x = torch.randn(coo.n, device=cuda, dtype=dt)
+    xh = x.cpu().pin_memory()
+    sets = [torch.from_numpy(s * np.asarray(coo.val)).to(cuda, dt) for s in (1.0, -0.5, 0.25)]
+    want = []
+    for v in sets:
+        plan.upload().set_values(v)
+        want.append(plan.spmv(x).cpu())
+    big = torch.randn(4096, 4096, device=cuda)
+    yhs = [torch.empty_like(want[0]).pin_memory() for _ in range(9)]
+    for yh in yhs:
+        yh.fill_(float("nan"))
+    for i, yh in enumerate(yhs):
+        big = big @ big * 1e-4  # the update waits its turn on the caller's stream
+        plan.set_values(sets[i % 3])
+        _call(plan, xh, yh, 1)
+    torch.cuda.synchronize()
+    for i, yh in enumerate(yhs):
+        assert torch.equal(yh, want[i % 3]), i
