@@ -440,7 +440,7 @@ class Plan:
                       stream=None):
         """``adjoint`` with the value gradient in input order (the caller's
         nonzeros): returns (gx, gin), None for an output not wanted.  The
-        first call uploads the nonzeros' rows and columns."""
+        first call gathers the nonzeros' rows and columns on the device."""
         import torch
         self.upload(stream)
         self._check_dev(g, x)

@@ -1190,20 +1190,29 @@ cbspmv_status cbspmv_grad_vals(cbspmv_plan *p, const void *g, const void *x,
 
 namespace {
 // The rows and columns of the input nonzeros on the device (the caller's
-// order), uploaded by the first call that needs them.
+// order), gathered there from the stored values' by the first call that needs
+// them.
 cbspmv_status ensure_input_coords(cbspmv_plan *p, cudaStream_t st) {
     std::lock_guard<std::mutex> lock(p->in_mu);
     if (p->in_ready) return CBSPMV_OK;
-    const cb::DeviceLayout &L = p->A.lay;
-    const size_t nnz = (size_t)p->host.nnz;
-    std::vector<int32_t> row(nnz), col(nnz);
-    for (size_t i = 0; i < nnz; ++i) {
-        row[i] = L.val_row[(size_t)L.input_slot[i]];
-        col[i] = L.val_col[(size_t)L.input_slot[i]];
+    const std::vector<int64_t> &slots = p->A.lay.input_slot;
+    const int64_t nnz = p->host.nnz;
+    int64_t *d_slot = nullptr;
+    cudaError_t e = cudaSuccess;
+    if (nnz > 0) {
+        const size_t bytes = (size_t)nnz * sizeof(int32_t);
+        e = cudaMalloc((void **)&d_slot, 2 * bytes);
+        if (e == cudaSuccess && !p->in_row) e = cudaMalloc((void **)&p->in_row, bytes);
+        if (e == cudaSuccess && !p->in_col) e = cudaMalloc((void **)&p->in_col, bytes);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(d_slot, slots.data(), 2 * bytes, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess)
+            e = cb::launch_input_coords(nnz, d_slot, p->A.val_row, p->A.val_col, p->in_row,
+                                        p->in_col, st);
     }
-    if (!p->in_row) CB_CUDA(upload_vec(row, &p->in_row, st), "upload input coordinates");
-    if (!p->in_col) CB_CUDA(upload_vec(col, &p->in_col, st), "upload input coordinates");
-    CB_CUDA(cudaStreamSynchronize(st), "upload input coordinates");
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (d_slot) cudaFree(d_slot);
+    if (e != cudaSuccess) return cuda_fail(e, "gather input coordinates");
     p->in_ready = true;
     return CBSPMV_OK;
 }

@@ -738,6 +738,19 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// Row and column of every input nonzero: those of its stored value.  Once a
+// plan; scattered 4-byte reads.
+__global__ void __launch_bounds__(256)
+    cb_input_coords_kernel(int64_t nnz, const int64_t *__restrict__ slot,
+                           const int32_t *__restrict__ vrow, const int32_t *__restrict__ vcol,
+                           int32_t *__restrict__ row, int32_t *__restrict__ col) {
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= nnz) return;
+    const int64_t v = slot[i];
+    row[i] = v < 0 ? -1 : vrow[v];
+    col[i] = v < 0 ? -1 : vcol[v];
+}
+
 template <typename T, int BS, int CH>
 cudaError_t launch_chunk(const DevLayout &d, const void *x, void *y, int nrhs,
                          int64_t ldx, int64_t ldy, cudaStream_t stream) {
@@ -1121,6 +1134,16 @@ cudaError_t launch_set_values(int f32, const ValueSide &a, const ValueSide &t, c
     else
         cb_set_values_kernel<double><<<(unsigned)b3, 256, 0, stream>>>(
             a, t, b0, b1, b2, static_cast<const double *>(in));
+    note_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_input_coords(int64_t nnz, const int64_t *slot, const int32_t *vrow,
+                                const int32_t *vcol, int32_t *row, int32_t *col,
+                                cudaStream_t stream) {
+    if (nnz == 0) return cudaSuccess;
+    cb_input_coords_kernel<<<(unsigned)((nnz + 255) / 256), 256, 0, stream>>>(nnz, slot, vrow,
+                                                                              vcol, row, col);
     note_launch();
     return cudaGetLastError();
 }

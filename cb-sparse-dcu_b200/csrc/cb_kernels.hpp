@@ -263,6 +263,11 @@ struct ValueSide {
 cudaError_t launch_set_values(int f32, const ValueSide &a, const ValueSide &t, const void *in,
                               cudaStream_t stream);
 
+// row[i], col[i] = vrow[slot[i]], vcol[slot[i]] for i < nnz.
+cudaError_t launch_input_coords(int64_t nnz, const int64_t *slot, const int32_t *vrow,
+                                const int32_t *vcol, int32_t *row, int32_t *col,
+                                cudaStream_t stream);
+
 // gvals[v] = sum_j g[row_v * ldg + j] * x[col_v * ldx + j] (0 when the slot
 // has no row or column)
 cudaError_t launch_grad_vals(int f32, int64_t nvals, const int32_t *vrow,

@@ -252,9 +252,9 @@ cbspmv_status cbspmv_adjoint(cbspmv_plan *plan, const void *g, const void *x,
 
 /* cbspmv_adjoint with the value gradient in the caller's input order: gin[k]
  * is the gradient of input nonzero k (every input is summed into exactly one
- * stored value, so it is that value's gradient).  The first call uploads the
- * input nonzeros' rows and columns (and waits for it), so make it before
- * capturing one. */
+ * stored value, so it is that value's gradient).  The first call gathers the
+ * input nonzeros' rows and columns on the device (and waits for it), so make
+ * it before capturing one. */
 cbspmv_status cbspmv_adjoint_input(cbspmv_plan *plan, const void *g, const void *x,
                              void *gx, void *gin, int nrhs, int64_t ldg,
                              int64_t ldx, int64_t ldgx, void *stream);
