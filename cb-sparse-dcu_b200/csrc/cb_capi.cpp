@@ -248,10 +248,10 @@ cbspmv_status upload_side(DevSide &s, cudaStream_t st) {
     CB_CUDA(upload_vec(L.block_cols, &s.block_cols, st), "upload gather list");
     s.one_source = !L.unit && (int64_t)L.vsrc.size() == L.nvals &&
                    (int64_t)L.vsrc_ptr.size() == L.nvals + 1;
+    const size_t vsz = L.f32 ? 4 : 8;
     for (int64_t v = 0; s.one_source && v < L.nvals; ++v)
-        s.one_source = L.vsrc_ptr[(size_t)v] == v;
+        s.one_source = L.vsrc_ptr[(size_t)v] == v && L.val_off[(size_t)v] + vsz <= L.payload.size();
     if (s.one_source) {  // sources and offsets in payload order (ValueSide)
-        const size_t vsz = L.f32 ? 4 : 8;
         std::vector<int32_t> at(L.payload.size() / vsz, -1);
         for (size_t v = 0; v < L.vsrc.size(); ++v) at[L.val_off[v] / vsz] = (int32_t)v;
         std::vector<int32_t> src;

@@ -269,16 +269,16 @@ std::string build_rowseg(const DeviceLayout &L, int64_t warps, RowSegHost &R) {
     // stored value v sits at payload offset val_off[v] (absent from plans
     // loaded from SpMV-only files, which take no new values)
     if (!unit && (int64_t)L.val_off.size() == L.nvals) {
-        std::vector<std::pair<int64_t, int32_t>> by_off((size_t)nv);
-        for (int64_t k = 0; k < nv; ++k) by_off[(size_t)k] = {eoff[(size_t)k], epos[(size_t)k]};
-        std::sort(by_off.begin(), by_off.end());
+        // (values sit at multiples of their size; a table over the payload:
+        // sorting the entries' offsets and searching them took 300 of 590 ms
+        // of the build of 2.4 M entries)
+        std::vector<int32_t> at(L.payload.size() / (size_t)vsz, -1);
+        for (int64_t k = 0; k < nv; ++k) at[(size_t)(eoff[(size_t)k] / vsz)] = epos[(size_t)k];
         R.vpos.resize((size_t)L.nvals);
+        // (a DENSE slot outside the valid columns or rows has no entry: -1)
         for (int64_t v = 0; v < L.nvals; ++v) {
-            const int64_t off = (int64_t)L.val_off[v];
-            auto it = std::lower_bound(by_off.begin(), by_off.end(),
-                                       std::make_pair(off, INT32_MIN));
-            // a DENSE slot outside the valid columns or rows has no entry
-            R.vpos[(size_t)v] = it != by_off.end() && it->first == off ? it->second : -1;
+            const uint64_t i = L.val_off[(size_t)v] / (uint64_t)vsz;
+            R.vpos[(size_t)v] = i < at.size() ? at[(size_t)i] : -1;
         }
     }
     R.alg_bytes = L.alg_bytes;
