@@ -10,6 +10,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <future>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <numeric>
@@ -594,6 +595,33 @@ cbspmv_status pipe_scratch(HostPipe &q, const DevSide &s, int nrhs) {
     return CBSPMV_OK;
 }
 
+cbspmv_status upload_plan(cbspmv_plan *p, cudaStream_t st) {
+    CB_CUDA(cudaGetDevice(&p->device), "cudaGetDevice");
+    if (!p->herr) {
+        CB_CUDA(cudaHostAlloc((void **)&p->herr, 16, cudaHostAllocMapped), "allocate error words");
+        std::memset(p->herr, 0, 16);
+        CB_CUDA(cudaHostGetDevicePointer((void **)&p->derr, p->herr, 0), "map error words");
+    }
+    cbspmv_status rc = upload_side(p->A, st);
+    if (!rc) rc = upload_partition(p->A, p->opts.kernel, st);
+    if (!rc) rc = upload_patterns(p->A, p->host, st);
+    if (!rc) rc = upload_rowseg(p->A, p->opts.kernel, st);
+    if (!rc && !p->spmv_only) rc = upload_balanced(p->A, p->host, p->opts.kernel, st);
+    if (!rc && p->has_t) rc = upload_side(p->AT, st);
+    if (!rc && p->has_t) rc = upload_partition(p->AT, p->opts.kernel, st);
+    if (!rc && p->has_t) rc = upload_rowseg(p->AT, p->opts.kernel, st);
+    p->A.d.err = p->derr;
+    p->AT.d.err = p->derr + 1;
+    if (rc) {
+        p->A.release();
+        p->AT.release();
+        return rc;
+    }
+    CB_CUDA(cudaStreamSynchronize(st), "upload");
+    p->uploaded = true;
+    return CBSPMV_OK;
+}
+
 cb::BuildOpts to_build(const cbspmv_opts &o) {
     cb::BuildOpts b;
     b.bs = o.block_size;
@@ -800,31 +828,15 @@ cbspmv_status cbspmv_plan_load(const char *path, cbspmv_plan **out) {
 cbspmv_status cbspmv_upload(cbspmv_plan *p, void *stream) {
     if (!p) return fail(CBSPMV_ERR_INVALID, "null plan");
     if (p->uploaded) return CBSPMV_OK;
-    cudaStream_t st = (cudaStream_t)stream;
-    CB_CUDA(cudaGetDevice(&p->device), "cudaGetDevice");
-    if (!p->herr) {
-        CB_CUDA(cudaHostAlloc((void **)&p->herr, 16, cudaHostAllocMapped), "allocate error words");
-        std::memset(p->herr, 0, 16);
-        CB_CUDA(cudaHostGetDevicePointer((void **)&p->derr, p->herr, 0), "map error words");
-    }
-    cbspmv_status rc = upload_side(p->A, st);
-    if (!rc) rc = upload_partition(p->A, p->opts.kernel, st);
-    if (!rc) rc = upload_patterns(p->A, p->host, st);
-    if (!rc) rc = upload_rowseg(p->A, p->opts.kernel, st);
-    if (!rc && !p->spmv_only) rc = upload_balanced(p->A, p->host, p->opts.kernel, st);
-    if (!rc && p->has_t) rc = upload_side(p->AT, st);
-    if (!rc && p->has_t) rc = upload_partition(p->AT, p->opts.kernel, st);
-    if (!rc && p->has_t) rc = upload_rowseg(p->AT, p->opts.kernel, st);
-    p->A.d.err = p->derr;
-    p->AT.d.err = p->derr + 1;
-    if (rc) {
+    try {
+        return upload_plan(p, (cudaStream_t)stream);
+    } catch (const std::bad_alloc &) {
+        // (copies out of vectors that are gone may still be under way)
+        cudaStreamSynchronize((cudaStream_t)stream);
         p->A.release();
         p->AT.release();
-        return rc;
+        return fail(CBSPMV_ERR_ALLOC, "out of host memory while uploading");
     }
-    CB_CUDA(cudaStreamSynchronize(st), "upload");
-    p->uploaded = true;
-    return CBSPMV_OK;
 }
 
 cbspmv_status cbspmv_spmv(cbspmv_plan *p, const void *x, void *y, int nrhs,
@@ -1541,21 +1553,29 @@ int64_t export_balanced(const cbspmv_plan *p, const std::string &k, void *out) {
 
 int64_t cbspmv_export(const cbspmv_plan *p, const char *name, void *out) {
     if (!p || !name) return -1;
-    const std::string k(name);
-    if (k.rfind("bal_", 0) == 0) return p->spmv_only ? -1 : export_balanced(p, k, out);
-    if (!exportable(p, k)) return -1;
-    if (k.rfind("dev_", 0) == 0 || k.rfind("rs_", 0) == 0)
-        return export_device(p->A.lay, k, out);
-    return cb::export_array(p->host, k, out);
+    try {
+        const std::string k(name);
+        if (k.rfind("bal_", 0) == 0) return p->spmv_only ? -1 : export_balanced(p, k, out);
+        if (!exportable(p, k)) return -1;
+        if (k.rfind("dev_", 0) == 0 || k.rfind("rs_", 0) == 0)
+            return export_device(p->A.lay, k, out);
+        return cb::export_array(p->host, k, out);
+    } catch (const std::bad_alloc &) {
+        return -1;
+    }
 }
 
 int64_t cbspmv_export_t(const cbspmv_plan *p, const char *name, void *out) {
     if (!p || !name || !p->has_t) return -1;
-    const std::string k(name);
-    if (!exportable(p, k)) return -1;
-    if (k.rfind("dev_", 0) == 0 || k.rfind("rs_", 0) == 0)
-        return export_device(p->AT.lay, k, out);
-    return cb::export_array(p->host_t, k, out);
+    try {
+        const std::string k(name);
+        if (!exportable(p, k)) return -1;
+        if (k.rfind("dev_", 0) == 0 || k.rfind("rs_", 0) == 0)
+            return export_device(p->AT.lay, k, out);
+        return cb::export_array(p->host_t, k, out);
+    } catch (const std::bad_alloc &) {
+        return -1;
+    }
 }
 
 void cbspmv_export_scalars(const cbspmv_plan *p, int transpose, int64_t *out12,
@@ -1807,12 +1827,8 @@ cbspmv_status batch_one(cbspmv_batch *b, cudaStream_t st) {
     return e == cudaSuccess ? CBSPMV_OK : cuda_fail(e, "batch launch");
 }
 
-}  // namespace
-
-extern "C" {
-
-cbspmv_status cbspmv_batch_create(cbspmv_plan *const *plans, int count, const int *nrhs,
-                                  cbspmv_batch **out) {
+cbspmv_status batch_create(cbspmv_plan *const *plans, int count, const int *nrhs,
+                           cbspmv_batch **out) {
     if (!plans || !nrhs || !out || count < 1)
         return fail(CBSPMV_ERR_INVALID, "batch needs count >= 1 plans and nrhs values");
     *out = nullptr;
@@ -1829,17 +1845,14 @@ cbspmv_status cbspmv_batch_create(cbspmv_plan *const *plans, int count, const in
             return fail(CBSPMV_ERR_INVALID, "batch plans must share block size and value type");
         if (nrhs[k] < 1) return fail(CBSPMV_ERR_INVALID, "nrhs must be >= 1");
     }
-    cbspmv_batch *b = new (std::nothrow) cbspmv_batch();
-    if (!b) return fail(CBSPMV_ERR_ALLOC, "out of host memory");
+    std::unique_ptr<cbspmv_batch> hold(new cbspmv_batch());
+    cbspmv_batch *const b = hold.get();
     b->bs = plans[0]->opts.block_size;
     b->f32 = plans[0]->opts.value_type == CBSPMV_F32;
     b->device = dev;
     for (int k = 0; k < count; ++k) {
         cbspmv_status rc = ensure_partials(plans[k]->A, nrhs[k], vsize(plans[k]));
-        if (rc) {
-            delete b;
-            return rc;
-        }
+        if (rc) return rc;
         b->tile_cap = std::max(b->tile_cap, plans[k]->A.d.mcap);
     }
     std::vector<int64_t> toff(1, 0);
@@ -1924,18 +1937,25 @@ cbspmv_status cbspmv_batch_create(cbspmv_plan *const *plans, int count, const in
         std::memset(b->herr, 0, 16);
         e = cudaHostGetDevicePointer((void **)&b->derr, b->herr, 0);
     }
-    if (e != cudaSuccess) {
-        delete b;
-        return cuda_fail(e, "allocate batch tables");
-    }
+    if (e != cudaSuccess) return cuda_fail(e, "allocate batch tables");
     cbspmv_status rc = batch_rowseg_setup(b, nrhs);
     if (!rc) rc = batch_scratch(b);
-    if (rc) {
-        delete b;
-        return rc;
-    }
-    *out = b;
+    if (rc) return rc;
+    *out = hold.release();
     return CBSPMV_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+cbspmv_status cbspmv_batch_create(cbspmv_plan *const *plans, int count, const int *nrhs,
+                                  cbspmv_batch **out) {
+    try {
+        return batch_create(plans, count, nrhs, out);
+    } catch (const std::bad_alloc &) {
+        return fail(CBSPMV_ERR_ALLOC, "out of host memory while building a batch");
+    }
 }
 
 cbspmv_status cbspmv_batch_bind(cbspmv_batch *b, const void *const *x, void *const *y,

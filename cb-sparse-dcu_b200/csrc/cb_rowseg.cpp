@@ -1,6 +1,8 @@
 // Host build of the row-segment stream (layout in cb_rowseg.hpp).
 #include "cb_rowseg.hpp"
 
+#include <omp.h>
+
 #include <algorithm>
 #include <climits>
 #include <cstring>
@@ -221,27 +223,33 @@ std::string build_rowseg(const DeviceLayout &L, int64_t warps, RowSegHost &R) {
     R.W = (int32_t)W;
     R.wbase.assign((size_t)G, 0);
     R.wlen.assign((size_t)G, 0);
-    // (threads only where the sorts outweigh a parallel region's start)
-#pragma omp parallel if (nv >= (int64_t(1) << 22))
+    // (threads only where the sorts outweigh a parallel region's start; their
+    // buffers are allocated before it, since nothing may throw out of it)
+    auto first_entry = [&](int64_t b) { return std::min(nv, b * nseg / G * M * C); };
+    size_t most = 0;  // entries of a CTA
+    for (int64_t b = 0; b < G; ++b)
+        most = std::max(most, (size_t)(first_entry(b + 1) - first_entry(b)));
+    const int threads = nv >= (int64_t(1) << 22) ? omp_get_max_threads() : 1;
+    std::vector<int32_t> all_cols(most * (size_t)threads), all_q(most * (size_t)threads);
+#pragma omp parallel num_threads(threads)
     {
-        std::vector<int32_t> cols;
-        std::vector<size_t> q;  // candidate first entries, their scores increasing
+        int32_t *const cols = all_cols.data() + most * (size_t)omp_get_thread_num();
+        // candidate first entries, their scores increasing
+        int32_t *const q = all_q.data() + most * (size_t)omp_get_thread_num();
 #pragma omp for schedule(dynamic, 1)
         for (int64_t b = 0; b < G; ++b) {
-            const int64_t s0 = b * nseg / G, s1 = (b + 1) * nseg / G;
-            const int64_t e0 = std::min(nv, s0 * M * C), e1 = std::min(nv, s1 * M * C);
+            const int64_t e0 = first_entry(b), e1 = first_entry(b + 1);
             if (e0 >= e1) continue;
-            cols.clear();
-            for (int64_t e = e0; e < e1; ++e) cols.push_back(ecol[order[(size_t)e]]);
-            std::sort(cols.begin(), cols.end());
-            auto score = [&](size_t i) { return kRsSector * (int64_t)i - vsz * cols[i]; };
-            q.clear();
-            size_t qh = 0;
+            const int32_t count = (int32_t)(e1 - e0);
+            for (int64_t e = e0; e < e1; ++e) cols[e - e0] = ecol[order[(size_t)e]];
+            std::sort(cols, cols + count);
+            auto score = [&](int32_t i) { return kRsSector * i - vsz * cols[i]; };
+            int32_t qh = 0, qt = 0;  // q[qh .. qt)
             int64_t best = 0;
             int32_t wb = 0, we = 0;  // the window's columns [wb, we)
-            for (size_t hi = 0; hi < cols.size(); ++hi) {
-                while (q.size() > qh && score(q.back()) >= score(hi)) q.pop_back();
-                q.push_back(hi);
+            for (int32_t hi = 0; hi < count; ++hi) {
+                while (qt > qh && score(q[qt - 1]) >= score(hi)) --qt;
+                q[qt++] = hi;
                 // (the window's first column moves down to a multiple of kRsWinAlign)
                 while (cols[hi] - (cols[q[qh]] & ~(kRsWinAlign - 1)) >= W) ++qh;
                 const int64_t gain = score(hi) - score(q[qh]) + kRsSector - vsz;
