@@ -305,20 +305,26 @@ cbspmv_status upload_side(DevSide &s, cudaStream_t st) {
     return CBSPMV_OK;
 }
 
-// The streaming kernel's per-warp tile ranges for this device's grid, and the
-// multi-right-hand-side kernel's tile buffer size.
+// The streaming kernel's per-warp tile ranges for this device's grid, when the
+// plan's kernel option (as s.d.kernel) allows that kernel.
+cbspmv_status upload_stream_ranges(DevSide &s, cudaStream_t st) {
+    const int64_t warps = s.wpart ? 0 : cb::stream_warps(s.d);
+    if (warps <= 0) return CBSPMV_OK;  // the direct kernel runs single vectors
+    const std::vector<uint32_t> part = cb::partition_tiles(s.lay, warps);
+    CB_CUDA(upload_vec(part, &s.wpart, st), "upload tile partition");
+    s.d.wpart = s.wpart;
+    s.d.nwarps = warps;
+    return CBSPMV_OK;
+}
+
+// Those ranges, and the multi-right-hand-side kernel's tile buffer size.
 cbspmv_status upload_partition(DevSide &s, int kernel, cudaStream_t st) {
     // the streaming partition whenever the layout allows that kernel, so a
     // later kernel choice (cbspmv_autotune) needs no new upload
     s.d.kernel = kernel == 0 || kernel == 1 ? kernel : 1;
-    const int64_t warps = cb::stream_warps(s.d);
+    const cbspmv_status rc = upload_stream_ranges(s, st);
     s.d.kernel = kernel;
-    if (warps > 0) {  // else the direct kernel runs single vectors
-        const std::vector<uint32_t> part = cb::partition_tiles(s.lay, warps);
-        CB_CUDA(upload_vec(part, &s.wpart, st), "upload tile partition");
-        s.d.wpart = s.wpart;
-        s.d.nwarps = warps;
-    }
+    if (rc) return rc;
     const int64_t nt = (int64_t)s.lay.tiles.size();
     if (nt > 0) {  // the direct kernel's block-row units
         const std::vector<uint32_t> du =
@@ -428,6 +434,16 @@ cbspmv_status upload_rowseg(DevSide &s, int kernel, cudaStream_t st) {
     d.unit = R.unit;
     s.rs_bytes = (int64_t)(R.chunks.size() + 4 * (R.meta.size() + R.spans.size() +
                                                   R.rowmap.size() + R.empty.size()));
+    if (cb::rowseg_tiles_faster(s.lay, R)) {
+        s.d.tiles_faster = 1;
+        if (cbspmv_status rc = upload_stream_ranges(s, st)) return rc;
+        // (where the tiles are too large for the streaming kernel, the direct
+        // one or the stream; n = 400000, 40% of the rows a band, unit values:
+        // 72 and 63 us FP64, 50 and 55 FP32, and with 32 x 32 blocks 55 and
+        // 63, 58 and 55)
+        s.d.tiles_faster =
+            s.d.wpart || (s.lay.unit && (s.lay.f32 != 0) == (s.lay.bs == 16));
+    }
     s.rs_nspan = R.spans.size() / 4;
     s.rs_cinfo = std::move(R.cinfo);
     s.rs_empty = std::move(R.empty);
@@ -1517,6 +1533,8 @@ int64_t export_device(const cb::DeviceLayout &L, const std::string &k, void *out
         if (f == "vpos") return raw(R.vpos.data(), R.vpos.size() * 4, 4);
         if (f == "wbase") return raw(R.wbase.data(), R.wbase.size() * 4, 4);
         if (f == "wlen") return raw(R.wlen.data(), R.wlen.size() * 4, 4);
+        const int32_t tiles = cb::rowseg_tiles_faster(L, R);
+        if (f == "tiles") return raw(&tiles, 4, 4);
     }
     return -1;
 }

@@ -833,7 +833,7 @@ bool use_stream(const DevLayout &d) {
     if (d.kernel == 1) return true;
     if (d.kernel >= 2) return false;
     if (d.small_direct) return false;
-    return d.coo_share >= 0.5;
+    return d.tiles_faster || d.coo_share >= 0.5;
 }
 
 template <typename T, int LP>
@@ -869,18 +869,19 @@ bool use_pattern(const DevLayout &d) {
 // Pattern reuse and the balanced schedule (plans built with row_owned = 0, the
 // reference's non-row-owned mode) take one right-hand side of unit stride.
 // The row-segment stream: when chosen, and the automatic choice except in
-// the reference's small-direct case.  It stores up to 4 bytes an entry
-// more than CSR and DENSE blocks do, but has no work per block: on
-// stencils (FP64, 3 unknowns a node) 24 us against the direct kernel's 46
-// at n = 98304 and 5.7 against 17 at n = 3000, on bands of 129 19 against
-// 43, on a dense 2000 x 2000 matrix 16 against 69 (the streaming kernel:
-// 35, 16, 20 and 30); FP32 and 32 x 32 blocks likewise
+// the reference's small-direct case and, for one right-hand side, where
+// rowseg_tiles_faster holds.  It reads up to 4 bytes an entry more than CSR
+// and DENSE blocks hold, but has no work per block: device times on stencils
+// (FP64, 3 unknowns a node, n = 98304) 23 us against the direct kernel's 46
+// and the streaming kernel's 35, on bands of 129 18 against 44 and 20, on a
+// dense 2000 x 2000 matrix 16 against 118 and 30; FP32 19, 30 and 29; 14, 27
+// and 17; 13, 50 and 21.
 int kernel_for(const DevLayout &d, int nrhs, int64_t ldx, int64_t ldy) {
     const bool one = nrhs == 1 && ldx == 1 && ldy == 1;
     if (one && use_pattern(d)) return 4;
     if (one && d.bal.rows && (d.kernel == 6 || d.kernel == 0)) return 6;
-    if (d.rs.chunks &&
-        (d.kernel == 5 || (d.kernel == 0 && !d.small_direct && !use_pattern(d))))
+    if (d.rs.chunks && (d.kernel == 5 || (d.kernel == 0 && !d.small_direct && !use_pattern(d) &&
+                                          !(one && d.tiles_faster))))
         return 5;
     if (one && use_stream(d)) return 1;
     return nrhs > 1 || d.kernel == 3 || d.kernel == 4 ? 3 : 2;

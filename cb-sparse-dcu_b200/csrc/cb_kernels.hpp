@@ -81,6 +81,9 @@ struct DevLayout {
     RowSegDev rs;                     // row-segment stream (kernel 5)
     BalancedDev bal;                  // balanced schedule (kernel 6; row_owned = 0)
     double coo_share = 1.0;
+    int tiles_faster = 0;             // automatic, one right-hand side: the streaming or
+                                      // direct kernel, not row segments
+                                      // (rowseg_tiles_faster)
     const uint32_t *wpart = nullptr;  // streaming: per-warp tile ranges
     int64_t nwarps = 0;               // streaming: warps of the launch
     uint32_t pay16_end = 0;           // payload size in 16-byte units

@@ -113,6 +113,40 @@ void tile_entries(const DeviceLayout &L, std::vector<int32_t> &erow, std::vector
     }
 }
 
+// The stream gives every CTA the same number of entries and reads 4 bytes of
+// index for each.  That loses to the tiles in two cases (device times, the
+// tiles first):
+//   * uneven scatter: the CTAs of a region of scattered rows, with no window,
+//     end last, where other rows are bands in DENSE blocks.  Unit values,
+//     16 x 16 blocks, 15% of the rows a band of 49: n = 150000 11.5 and 12.6
+//     us, n = 300000 19.2 and 21.3, n = 1000000 54 and 64, but n = 100000 9.0
+//     and 9.0; 32 x 32 blocks n = 1000000 53 and 64, but n = 150000 18.3 and
+//     12.6; FP32 values, 16 x 16 blocks, n = 1000000 58 and 64, but n = 300000
+//     21.7 and 20.9.  FP64 values: never (n = 1000000 70 and 68).  Nor with
+//     few entries a tile, which bring the work per tile back: 10% of the rows
+//     a band, n = 2000000, 137 entries a tile, 83 and 76 (n = 1000000 above:
+//     213 a tile).
+//   * unit values in DENSE blocks, a bit each: bands of 129, n = 150000 22 and
+//     43 us, n = 40000 10.4 and 14.2, but n = 20000 9.8 and 9.5; bands of 49
+//     (a third of the entries in DENSE blocks), n = 300000 26 and 33, but
+//     n = 80000 11.7 and 11.9.
+bool rowseg_tiles_faster(const DeviceLayout &L, const RowSegHost &R) {
+    int64_t dense = 0, all = 0;
+    for (const TileDesc &t : L.tiles) all += t.coo_entries;
+    for (const BlockDesc &b : L.blocks) {
+        if (meta_type(b.meta) == 0) continue;
+        all += meta_nnz(b.meta);
+        if (meta_type(b.meta) != 1) dense += meta_nnz(b.meta);
+    }
+    if (dense == 0 || all < 192 * (int64_t)L.tiles.size()) return false;
+    // (nearly) all of the worst CTA's entries scattered, far fewer on average
+    const bool uneven = 10 * R.cta_out >= 9 * R.cta_entries && 10 * R.mean_out <= 7 * R.cta_out;
+    if (L.unit)
+        return (uneven && R.cta_out >= (L.bs == 16 ? 12000 : 60000)) ||
+               (10 * dense >= 3 * all && R.cta_entries >= 30000);
+    return L.f32 && L.bs == 16 && uneven && R.cta_out >= 60000;
+}
+
 std::string build_rowseg(const DeviceLayout &L, int64_t warps, RowSegHost &R) {
     if (!rowseg_applies(L)) return "the layout does not take the row-segment stream";
     const int64_t m = L.m, C = rs_chunk_entries();
@@ -229,6 +263,7 @@ std::string build_rowseg(const DeviceLayout &L, int64_t warps, RowSegHost &R) {
     size_t most = 0;  // entries of a CTA
     for (int64_t b = 0; b < G; ++b)
         most = std::max(most, (size_t)(first_entry(b + 1) - first_entry(b)));
+    std::vector<int64_t> outs((size_t)G, 0);  // entries outside the window
     const int threads = nv >= (int64_t(1) << 22) ? omp_get_max_threads() : 1;
     std::vector<int32_t> all_cols(most * (size_t)threads), all_q(most * (size_t)threads);
 #pragma omp parallel num_threads(threads)
@@ -261,9 +296,11 @@ std::string build_rowseg(const DeviceLayout &L, int64_t warps, RowSegHost &R) {
             }
             R.wbase[(size_t)b] = wb;
             R.wlen[(size_t)b] = we - wb;
+            outs[(size_t)b] = count;
             for (int64_t e = e0; e < e1; ++e) {
                 const int32_t col = ecol[order[(size_t)e]];
                 if (col >= wb && col < we) {
+                    --outs[(size_t)b];
                     const int64_t c = e / C, i = e % C;
                     uint32_t word;
                     std::memcpy(&word, R.chunks.data() + c * CB + 4 * i, 4);
@@ -273,6 +310,12 @@ std::string build_rowseg(const DeviceLayout &L, int64_t warps, RowSegHost &R) {
             }
         }
     }
+    R.cta_entries = (int64_t)most;
+    for (int64_t o : outs) {
+        R.cta_out = std::max(R.cta_out, o);
+        R.mean_out += o;
+    }
+    R.mean_out /= G;
     // per stored value (device order) its stream entry, for value updates:
     // stored value v sits at payload offset val_off[v] (absent from plans
     // loaded from SpMV-only files, which take no new values)

@@ -95,8 +95,15 @@ struct RowSegHost {
     std::vector<int32_t> empty;    // rows with no stored entry
     std::vector<int32_t> vpos;     // per stored value (device order): its stream entry,
                                    // or empty without per-value offsets
+    // entries of the largest CTA, and outside their CTA's window: of the CTA
+    // with most, and of the mean one
+    int64_t cta_entries = 0, cta_out = 0, mean_out = 0;
     int64_t alg_bytes = 0;
 };
+
+// Whether one right-hand side runs faster on the streaming tile kernel than on
+// the stream R of a layout with CSR or DENSE blocks.
+bool rowseg_tiles_faster(const DeviceLayout &L, const RowSegHost &R);
 
 // Whether the layout takes the row-segment stream: stored entries, columns
 // below 2^30, rows below 2^31 (CSR and DENSE blocks are expanded into

@@ -70,10 +70,13 @@ typedef struct cbspmv_opts {
                              cb-spmv-dcu.hpp:1431-1433), 5 row segments (the
                              stored entries sorted by row in chunks of 128,
                              summed per lane and joined by one scan; built
-                             at upload, and the automatic choice; keeps a
-                             second copy of the values on the device), 6 balanced (plans built with row_owned
-                             = 0 and stored values: the entries in the
-                             plan's block order, grouped as the reference's
+                             at upload, and the automatic choice but for one
+                             right-hand side on some large layouts with
+                             DENSE blocks, unit-valued ones most; keeps a
+                             second copy of the values on the device), 6
+                             balanced (plans built with row_owned = 0 and
+                             stored values: the entries in the plan's block
+                             order, grouped as the reference's
                              CTAs, added into y with atomics as its
                              non-row-owned mode does; the automatic choice
                              for one right-hand side on such plans); see
