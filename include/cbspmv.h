@@ -347,12 +347,13 @@ void cbspmv_debug_wait_polls(int64_t polls);
 /* Times the kernels that can run this plan for nrhs right-hand sides (one
  * vector: streaming when the layout allows it, direct, staged, and pattern
  * reuse, row segments and the balanced schedule when the plan has them;
- * several: the staged kernel and row segments) on scratch vectors, keeps
- * the fastest for later calls (the automatic choice where none beats it by
- * more than 0.3 us and 1%, which the timing does not tell apart) and returns
- * it in *kernel (1 to 6) with its mean time in *ms (either may be NULL).  The
- * plan must be uploaded; allocates and frees scratch device
- * memory and synchronizes `stream`.  No counterpart in the reference (its
+ * several: the staged kernel and row segments) on scratch vectors, by their
+ * device time (replays of a captured graph of launches, on a stream of its own
+ * after `stream`), keeps the fastest for later calls (the automatic choice
+ * where none beats it by more than 1%, which the timing does not tell apart)
+ * and returns it in *kernel (1 to 6) with its mean time in *ms (either may be
+ * NULL).  The plan must be uploaded; allocates and frees scratch device memory
+ * and waits for `stream`.  No counterpart in the reference (its
  * kernel choice is compile-time, cb-spmv-dcu.hpp:1428-1450). */
 cbspmv_status cbspmv_autotune(cbspmv_plan *plan, int nrhs, void *stream, int *kernel,
                               double *ms);

@@ -1,5 +1,6 @@
-"""The tuner's choice among kernels that launching bounds alike (GPU): the
-automatic choice, every time."""
+"""The tuner's choice among kernels of small products (GPU), which all take the
+host's time a launch when launched one by one: by their device time, the same
+every time (pattern reuse 2.6 us here, row segments 4.4)."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -7,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("f32", [False, True])
 @pytest.mark.parametrize("bs", [16, 32])
-def test_ties_go_to_the_automatic_choice(cuda, f32, bs):
+def test_small_products_are_told_apart(cuda, f32, bs):
     import cbspmv
     from test_gpu_spmv import _patterned
     plan = cbspmv.Plan(_patterned(), value_type=int(f32), block_size=bs)
