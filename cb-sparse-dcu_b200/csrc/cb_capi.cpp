@@ -79,8 +79,8 @@ struct DevSide {
     int32_t *val_row = nullptr, *val_col = nullptr;
     int32_t *pat[4] = {};  // pattern row_ptr, col_idx, output_ptr, output_rows
     // row-segment stream (kernel 5): chunks, segment meta, spans, counters,
-    // partial slots, rowmap, empty rows, value positions or entries' inputs, window bases, window lengths,
-    // exchange words
+    // partial slots, rowmap, empty rows, value positions or entries' inputs,
+    // window bases, window lengths, exchange words
     void *rs[11] = {};
     int64_t rs_bytes = 0;
     size_t rs_nspan = 0;
@@ -430,7 +430,6 @@ cbspmv_status upload_rowseg(DevSide &s, int kernel, cudaStream_t st) {
     d.W = std::max<int32_t>(1, *std::max_element(R.wlen.begin(), R.wlen.end()));
     d.wbase = static_cast<const int32_t *>(s.rs[8]);
     d.wlen = static_cast<const int32_t *>(s.rs[9]);
-    d.n = R.n;
     d.unit = R.unit;
     s.rs_bytes = (int64_t)(R.chunks.size() + 4 * (R.meta.size() + R.spans.size() +
                                                   R.rowmap.size() + R.empty.size()));

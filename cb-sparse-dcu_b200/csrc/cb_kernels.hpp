@@ -33,7 +33,6 @@ struct RowSegDev {
     int32_t G = 0, W = 0;             // CTAs of every launch; longest window (values)
     const int32_t *wbase = nullptr;   // per CTA: first column of its x window
     const int32_t *wlen = nullptr;    // per CTA: columns of its x window
-    int64_t n = 0;                    // columns (length of x)
     int unit = 0;                     // words only: every stored value is 1
 };
 

@@ -250,7 +250,7 @@ std::string build_rowseg(const DeviceLayout &L, int64_t warps, RowSegHost &R) {
     // saves its entries a 32-byte sector of L2 traffic each, so per CTA the
     // window of at most W columns with the largest saving minus cost (a
     // sliding minimum over its sorted columns), aligned down to kRsWinAlign
-    // columns; no window where every one costs more than it saves
+    // columns
     const int64_t G = std::max<int64_t>(1, std::max<int64_t>(warps, 1) / kRsWarps);
     const int64_t W = kRsWindowBytes / vsz;
     R.G = (int32_t)G;

@@ -26,12 +26,12 @@
 // y; either way results do not depend on timing.
 // Each CTA also holds a WINDOW of x in shared memory: wlen[b] consecutive
 // columns from wbase[b], at most kRsWindowBytes, chosen on the host as the one
-// that saves the most gather traffic over its own staging (none where every
-// window costs more than it saves); an entry whose column lies in its CTA's
-// window carries bit 30 and reads x from there (a shared-memory gather costs
-// a few wavefronts per warp where 32 scattered global loads cost 32 L1 tag
-// lookups).  The segments are assigned to CTAs for a grid of G CTAs fixed at
-// build time, so every launch uses that grid.
+// that saves the most gather traffic over its own staging (a few columns where
+// no longer one pays, none without entries); an entry whose column lies in its
+// CTA's window carries bit 30 and reads x from there (a shared-memory gather
+// costs a few wavefronts per warp where 32 scattered global loads cost 32 L1
+// tag lookups).  The segments are assigned to CTAs for a grid of G CTAs fixed
+// at build time, so every launch uses that grid.
 // Rows are counted as ORDINALS of the non-empty rows (rowmap maps them back
 // when some rows are empty; those rows are listed in `empty` and zeroed).
 // The entry count is padded to whole chunks with entries of value 0 on
@@ -120,10 +120,11 @@ void rowseg_cut(const std::vector<int32_t> &cinfo, const std::vector<int64_t> &c
                 int64_t seg0, int32_t tag, std::vector<int32_t> &meta,
                 std::vector<int32_t> &spans);
 
-// Builds the stream from the tiles' COO sections (row, column and value of
-// every entry) for `warps` resident warps (G = warps / kRsWarps CTAs); vpos only when the layout has its
-// per-value offsets (val_off).  Every plan of one matrix and value type gets
-// the same stream, so the same sums.  Returns "" or an error.
+// Builds the stream from the tiles (row, column and value of every entry of
+// their COO sections, CSR and DENSE blocks) for `warps` resident warps (G =
+// warps / kRsWarps CTAs); vpos only when the layout has its per-value offsets
+// (val_off).  Every plan of one matrix and value type gets the same stream, so
+// the same sums.  Returns "" or an error.
 std::string build_rowseg(const DeviceLayout &L, int64_t warps, RowSegHost &R);
 
 // The balanced (non-row-owned) schedule of a plan built with row_owned = 0:

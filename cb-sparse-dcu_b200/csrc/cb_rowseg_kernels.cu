@@ -24,9 +24,11 @@
 //     (reset at lanes holding a row start, its steps' lanes read off the
 //     ballots, ended once no row reaches further), carrying the chunk's last
 //     row into the next chunk.
-// Bound by instruction issue and the gathers outside the window; with the row
-// starts and the scan's flags shuffled instead, n = 1048576, mean 16, FP64
-// took 56.8 us instead of 49.5, n = 300007, FP32 18.1 instead of 15.7.
+// Bound by L1 (76% of its rate) and issue (63%) on large power-law matrices,
+// by issue (63%) on stencils, and by the latency of a warp's few chunks in a
+// row on mid-sized matrices (issue 52%, L1 49%).  Row starts and the scan's
+// flags from ballots instead of shuffles, with windows no longer than they
+// pay, took 13% off, n = 1048576, mean 16, FP64 and n = 300007, FP32.
 // The products of one row are added in entry order within a lane and in lane
 // order across lanes, fixed by the layout: results are bitwise reproducible
 // (the balanced schedule's atomics excepted).  The reference adds each entry
@@ -116,9 +118,10 @@ __device__ __forceinline__ void unpack(const float4 &v, float *o) {
 // back, has the row's sum (two addends: the same in either order) and empties
 // the word.  The value travels in the atomic, so no fence is needed: the
 // acquire-release counter below made each warp wait for all its stores of y
-// (8-10% of the warps' cycles on power-law matrices: n = 300007, FP32
-// 15.7 -> 14.4 us; 256 x 256 grid 6.0 -> 4.2; a batch of 32 114 -> 98).  A part with kEmpty's
-// bits, a NaN, goes in as the ordinary NaN.  Returns true with v the sum.
+// (8-10% of the warps' cycles on power-law matrices; device time without it
+// -8% at n = 300007, FP32, -30% on a 256 x 256 grid, -14% for a batch of 32).
+// A part with kEmpty's bits, a NaN, goes in as the ordinary NaN.  Returns true
+// with v the sum.
 template <typename T> struct RsBits;
 template <> struct RsBits<float> {
     using U = unsigned int;
@@ -772,9 +775,9 @@ __global__ void cb_balanced_values_kernel(const BalancedDev b, const uint8_t *__
 
 // Launches a kernel that begins with dev::behind_wait: its blocks are set up
 // while the launch before it drains, so a call in a solver's loop does not pay
-// the launch latency between its kernels.  Calls one after another, without
-// and with: 256 x 256 grid, FP64 6.1 and 5.1 us; n = 300007, FP32 18.2 and
-// 16.0; uniform A x and A^T y 30.8 and 27.9.  Such a kernel reads what a
+// the launch latency between its kernels.  Time a call, one after another,
+// without and with: 256 x 256 grid, FP64 6.1 and 5.1 us; n = 300007, FP32 18.2
+// and 16.0; uniform A x and A^T y 30.8 and 27.9.  Such a kernel reads what a
 // launch before it may have written (x, the stream's values) by coherent
 // volatile loads (ld_x, ld_stream, stage_window): one through the read-only
 // path (__ldg) could be moved before behind_wait and need not see those

@@ -17,8 +17,12 @@
  *     failure;
  *   - pointers are plain host or device addresses; streams are cudaStream_t
  *     passed as void* (0 = the legacy default stream);
- *   - a plan is immutable after upload; one plan may be executed on one
- *     stream at a time (its split-row scratch is shared by its launches).
+ *   - a plan is immutable after upload; its launches share its scratch (the
+ *     row-segment stream's exchange words, counters and slots, split rows'
+ *     partials), so no two may overlap: one plan runs on one stream at a
+ *     time.  Launches that did overlap can leave wrong rows in later calls
+ *     too.  (cbspmv_spmv_host_async and cbspmv_batch_run have scratch of
+ *     their own.)
  */
 #ifndef CBSPMV_H
 #define CBSPMV_H
@@ -202,8 +206,8 @@ cbspmv_status cbspmv_spmv(cbspmv_plan *plan, const void *x, void *y, int nrhs,
  * different streams, or from different plans -- race.  The looked-up address
  * is kept for the process: do not use this call after a device reset
  * (cudaDeviceReset) in the same process.  Plans whose kernel is the
- * row-segment stream need no scratch from the array (their span counters
- * and slots are the plan's own, allocated at upload). */
+ * row-segment stream need no scratch from the array (their exchange words,
+ * span counters and slots are the plan's own, allocated at upload). */
 cbspmv_status cbspmv_spmv_noalloc(cbspmv_plan *plan, const void *x, void *y,
                                   int nrhs, int64_t ldx, int64_t ldy,
                                   void *stream);
@@ -304,11 +308,12 @@ cbspmv_status cbspmv_info_get(const cbspmv_plan *plan, cbspmv_info *info);
  * dev_blocks (uint32 words), dev_payload (bytes) and dev_values (double, one
  * per stored slot) give the device layout itself; rs_sizes (nch, M, nseg,
  * nord, G, W), rs_chunks (bytes), rs_meta, rs_spans, rs_rowmap, rs_empty,
- * rs_vpos and rs_wbase (int32), each
- * followed by ":W", the row-segment stream as built for W resident warps
- * (-1 when the layout does not take it); bal_rows, bal_cols (uint32), bal_vals
- * (the value type) and bal_gstart (int64), the balanced schedule's stream
- * of a plan built with row_owned = 0 (-1 otherwise). */
+ * rs_vpos, rs_wbase, rs_wlen (int32) and rs_tiles (int32, one: 1 where the
+ * automatic choice for one right-hand side keeps the tiles), each followed by
+ * ":W", the row-segment stream as built for W resident warps (-1 when the
+ * layout does not take it, or out of host memory); bal_rows, bal_cols
+ * (uint32), bal_vals (the value type) and bal_gstart (int64), the balanced
+ * schedule's stream of a plan built with row_owned = 0 (-1 otherwise). */
 int64_t cbspmv_export(const cbspmv_plan *plan, const char *name, void *out);
 
 /* The same for the CB structure of A^T (plans built with want_transpose). */
