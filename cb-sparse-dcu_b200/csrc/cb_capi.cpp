@@ -67,8 +67,8 @@ struct DevSide {
     int64_t *ustart = nullptr;
     int partial_nrhs = 0;
     // partials that were too small for a later call: graphs captured before it
-    // and bound batches still use them.  Each is at least twice the one before,
-    // so together they are smaller than the one in use.
+    // still use them.  Each is at least twice the one before (while memory
+    // lasts), so together they are smaller than the one in use.
     void *old_partials[32] = {};
     int nold = 0;
     int64_t *vsrc_ptr = nullptr;
@@ -502,11 +502,21 @@ cbspmv_status upload_patterns(DevSide &s, const cb::HostCB &g, cudaStream_t st) 
 // the plan is destroyed (see DevSide::old_partials).
 cbspmv_status ensure_partials(DevSide &s, int nrhs, size_t vsz) {
     if (s.lay.slots == 0 || s.partial_nrhs >= nrhs) return CBSPMV_OK;
-    const int64_t want = std::min<int64_t>(std::max<int64_t>(nrhs, 2 * (int64_t)s.partial_nrhs),
-                                           INT32_MAX);
+    int64_t want = std::min<int64_t>(std::max<int64_t>(nrhs, 2 * (int64_t)s.partial_nrhs),
+                                     INT32_MAX);
+    const size_t each = (size_t)s.lay.slots * s.lay.bs * vsz;
     void *fresh = nullptr;
-    CB_CUDA(cudaMalloc(&fresh, (size_t)s.lay.slots * (size_t)want * s.lay.bs * vsz),
-            "allocate split-row partials");
+    cudaError_t e = cudaMalloc(&fresh, each * (size_t)want);
+    if (e == cudaErrorMemoryAllocation && want > nrhs) {  // no more than asked for
+        cudaGetLastError();
+        want = nrhs;
+        e = cudaMalloc(&fresh, each * (size_t)want);
+    }
+    CB_CUDA(e, "allocate split-row partials");
+    if (s.partials && s.nold == 32) {  // (only after many growths by less than twice)
+        cudaFree(fresh);
+        return fail(CBSPMV_ERR_ALLOC, "split-row partials grew too often");
+    }
     if (s.partials) s.old_partials[s.nold++] = s.partials;
     s.partials = fresh;
     s.partial_nrhs = (int)want;
