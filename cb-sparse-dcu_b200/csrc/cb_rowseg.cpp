@@ -264,7 +264,8 @@ std::string build_rowseg(const DeviceLayout &L, int64_t warps, RowSegHost &R) {
     for (int64_t b = 0; b < G; ++b)
         most = std::max(most, (size_t)(first_entry(b + 1) - first_entry(b)));
     std::vector<int64_t> outs((size_t)G, 0);  // entries outside the window
-    const int threads = nv >= (int64_t(1) << 22) ? omp_get_max_threads() : 1;
+    const int threads =
+        nv >= (int64_t(1) << 22) ? (int)std::min<int64_t>(omp_get_max_threads(), G) : 1;
     std::vector<int32_t> all_cols(most * (size_t)threads), all_q(most * (size_t)threads);
 #pragma omp parallel num_threads(threads)
     {
